@@ -196,6 +196,26 @@ def load_library() -> ctypes.CDLL:
     return lib
 
 
+_front = None
+_FRONT_FUNCTIONS = ("sdxlq_linear", "sdxlq_linear_grouped", "sdxlq_layer_norm", "sdxlq_quantize_act_int8",
+                    "sdxlq_quantize_act_fp8", "sdxlq_pack_weight_int8", "sdxlq_pack_weight_fp8")
+
+
+def load_front():
+    """The native front (csrc/torch_front.cpp), bound to the loaded library. It issues ordinary calls without
+    ctypes; calls it does not take (it answers None) are checked and issued by the Python code below."""
+    global _front
+    if _front is None:
+        lib = load_library()
+        if not os.path.exists(_build.FRONT):
+            raise CudaError(f"{_build.FRONT} is missing: build it first (build() of this package, or "
+                            "__graft_entry__.build())", STATUS_CUDA)
+        from . import _front as module
+        module.bind(*(ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in _FRONT_FUNCTIONS))
+        _front = module
+    return _front
+
+
 def valid_convrot_group_size(group_size: int) -> bool:
     """valid_convrot_group_size (src/cuda/int8_convrot.cu:489-496): power of four in 4..256."""
     if group_size < 4 or group_size > 256:
@@ -302,7 +322,9 @@ class Context:
     def __init__(self, device: int = 0, stream: Optional[torch.cuda.Stream] = None,
                  workspace_bytes: int = 0):
         self._lib = load_library()
+        self._front = load_front()
         self._handle = ctypes.c_void_p()
+        self.address = 0                       # of the sdxlq_context, for the native front
         self.device = device
         self.stream = stream
         stream_ptr = ctypes.c_void_p(stream.cuda_stream) if stream is not None else \
@@ -310,11 +332,13 @@ class Context:
         status = self._lib.sdxlq_context_create(device, stream_ptr, workspace_bytes, ctypes.byref(self._handle))
         if status != STATUS_OK:
             raise CudaError(f"sdxlq_context_create failed: {self._lib.sdxlq_status_string(status).decode()}", status)
+        self.address = self._handle.value
 
     def close(self) -> None:
         if getattr(self, "_handle", None) and self._handle.value:
             self._lib.sdxlq_context_destroy(self._handle)
             self._handle = ctypes.c_void_p()
+            self.address = 0
 
     def __del__(self):
         try:
@@ -374,6 +398,7 @@ class Ops:
     def __init__(self, context: Context, poison_outputs: bool = False):
         self.ctx = context
         self._lib = context._lib
+        self._front = getattr(context, "_front", None)
         # Tests set this: outputs this class allocates start as NaN, so that an element a kernel
         # failed to write cannot pass for a result left in recycled memory.
         self.poison_outputs = poison_outputs
@@ -423,6 +448,10 @@ class Ops:
         """`residual` folds the Ops::add_in_place that follows the projection in the reference's
         transformer block (src/cuda/unet.cpp:118, 132, 147) into the epilogue; pass out=residual to
         update the hidden state in place."""
+        y = self._front.linear(self.ctx.address, input, weight, bias, ACT_NONE, out, xq, xq_scales, acc_out, residual,
+                               y_amax, x_amax, self.poison_outputs)
+        if y is not None:
+            return y if y.__class__ is not int else self.ctx.raise_for(y)
         call = LinearCall(input, weight, bias, ACT_NONE, out, xq, xq_scales, acc_out, residual, y_amax, x_amax)
         desc = self._desc(call)
         self.ctx.raise_for(self._lib.sdxlq_linear(self.ctx.handle, ctypes.byref(desc)))
@@ -434,6 +463,10 @@ class Ops:
                           acc_out: Optional[torch.Tensor] = None,
                           out: Optional[torch.Tensor] = None, y_amax: Optional[torch.Tensor] = None,
                           x_amax: Optional[torch.Tensor] = None) -> torch.Tensor:
+        y = self._front.linear(self.ctx.address, input, weight, bias, activation, out, xq, xq_scales, acc_out, None,
+                               y_amax, x_amax, self.poison_outputs)
+        if y is not None:
+            return y if y.__class__ is not int else self.ctx.raise_for(y)
         call = LinearCall(input, weight, bias, int(activation), out, xq, xq_scales, acc_out, None, y_amax, x_amax)
         desc = self._desc(call)
         self.ctx.raise_for(self._lib.sdxlq_linear(self.ctx.handle, ctypes.byref(desc)))
@@ -447,6 +480,9 @@ class Ops:
         return array
 
     def linear_grouped(self, calls: Sequence[LinearCall]) -> list:
+        outputs = self._front.linear_grouped(self.ctx.address, calls, self.poison_outputs)
+        if outputs is not None:
+            return outputs if outputs.__class__ is not int else self.ctx.raise_for(outputs)
         array = self._desc_array(calls)
         self.ctx.raise_for(self._lib.sdxlq_linear_grouped(self.ctx.handle, array, len(calls)))
         return [call.y for call in calls]
@@ -475,6 +511,9 @@ class Ops:
     def layer_norm(self, input: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor,
                    epsilon: float = 1.0e-5, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Ops::layer_norm (include/sdxl/cuda/ops.hpp:39-42): FP16 in, FP16 out."""
+        y = self._front.layer_norm(self.ctx.address, input, weight, bias, epsilon, out, None)
+        if y is not None:
+            return y if y.__class__ is not int else self.ctx.raise_for(y)
         rows, width = self._layer_norm_check(input, weight, bias)
         y = out if out is not None else torch.empty_like(input)
         desc = _CLayerNormDesc(input.data_ptr(), rows, width, weight.data_ptr(), bias.data_ptr(), epsilon,
@@ -488,6 +527,9 @@ class Ops:
         returns (xq, xq_scales) in the form `consumer` (an INT8 or FP8 projection weight) wants, to be
         passed as linear(None, consumer, ..., xq=xq, xq_scales=xq_scales). Equal to quantising
         layer_norm(input) with quantize_int8 / quantize_fp8, without the FP16 tensor in between."""
+        pair = self._front.layer_norm(self.ctx.address, input, weight, bias, epsilon, None, consumer)
+        if pair is not None:
+            return pair if pair.__class__ is not int else self.ctx.raise_for(pair)
         rows, width = self._layer_norm_check(input, weight, bias)
         if consumer.k != width:
             raise CudaError("CUDA linear feature mismatch")
@@ -554,10 +596,16 @@ class Ops:
         if input.dtype != torch.float16 or fp8_type not in _TORCH_FP8:
             raise CudaError("FP8 activation quantization requires float16 input and an FP8 destination")
         source = input.contiguous()
-        q = torch.empty(source.shape, dtype=torch.uint8, device=source.device)
-        scale = torch.empty(1, dtype=torch.float32, device=source.device)
-        self.ctx.raise_for(self._lib.sdxlq_quantize_act_fp8(
-            self.ctx.handle, source.data_ptr(), source.numel(), int(fp8_type), q.data_ptr(), scale.data_ptr()))
+        pair = self._front.quantize_fp8(self.ctx.address, source, fp8_type)
+        if pair.__class__ is int:
+            self.ctx.raise_for(pair)
+        if pair is not None:
+            q, scale = pair
+        else:
+            q = torch.empty(source.shape, dtype=torch.uint8, device=source.device)
+            scale = torch.empty(1, dtype=torch.float32, device=source.device)
+            self.ctx.raise_for(self._lib.sdxlq_quantize_act_fp8(
+                self.ctx.handle, source.data_ptr(), source.numel(), int(fp8_type), q.data_ptr(), scale.data_ptr()))
         n = source.shape[0] if source.dim() == 2 else source.numel() // source.shape[-1]
         return Weight(q, ScalarType(fp8_type), n, source.shape[-1], scale, FP8ScaleMode.TensorWide)
 
@@ -574,6 +622,9 @@ class Ops:
         if input.dtype not in (torch.float16, torch.float32) or input.dim() < 2:
             raise CudaError("native INT8 linear received incompatible tensors")
         source = input.contiguous()
+        pair = self._front.quantize_int8(self.ctx.address, source, convrot_group_size, False)
+        if pair is not None:
+            return pair if pair.__class__ is not int else self.ctx.raise_for(pair)
         k = source.shape[-1]
         m = source.numel() // k
         xq = torch.empty(source.shape, dtype=torch.int8, device=source.device)
@@ -617,6 +668,12 @@ class Ops:
         if not prequantized and source.dtype not in (torch.float16, torch.float32):
             source = source.to(torch.float32)
         source = source.contiguous()
+        pair = None if prequantized else self._front.quantize_int8(self.ctx.address, source, group, True)
+        if pair.__class__ is int:
+            self.ctx.raise_for(pair)
+        if pair is not None:
+            return Weight(pair[0], ScalarType.Int8, rows, columns, pair[1], FP8ScaleMode.PerOutputChannel,
+                          FP8StorageLayout.RowMajorNK, group if use_convrot else 0)
         weight = torch.empty((rows, columns), dtype=torch.int8, device=source.device)
         if prequantized:
             scales = metadata.weight_scale.to(device=source.device, dtype=torch.float32).reshape(rows).contiguous()
@@ -648,6 +705,11 @@ class Ops:
             source = source.to(torch.float32)
             src_dtype = ScalarType.Float32
         source = source.contiguous()
+        pair = self._front.pack_fp8(self.ctx.address, source, src_dtype, options.format, options.scale_mode, options.layout)
+        if pair.__class__ is int:
+            self.ctx.raise_for(pair)
+        if pair is not None:
+            return Weight(pair[0], ScalarType(options.format), rows, columns, pair[1], options.scale_mode, options.layout)
         count = rows if options.scale_mode == FP8ScaleMode.PerOutputChannel else 1
         shape = (columns, rows) if options.layout == FP8StorageLayout.KMajorKN else (rows, columns)
         packed = torch.empty(shape, dtype=torch.uint8, device=source.device)

@@ -1,0 +1,62 @@
+"""The native front (csrc/torch_front.cpp) and the ctypes path issue the same calls: same bits for every form
+of argument, and the front hands over what it does not take, so that errors keep their messages."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+class _NoFront:
+    """Answers None to everything: the Python path runs."""
+
+    def __getattr__(self, name):
+        return lambda *arguments: None
+
+
+@pytest.mark.parametrize("dtype", ["int8", "e4m3", "f16"])
+@pytest.mark.parametrize("lead", [(5,), (2, 77), (1, 3, 7)])
+def test_front_and_python_path_agree(gpu, dtype, lead):
+    pkg, ctx, ops = gpu
+    slow = pkg.Ops(ctx, poison_outputs=True)
+    slow._front = _NoFront()
+    torch.manual_seed(3)
+    k, n = 256, 64
+    x = torch.randn(*lead, k, device="cuda").half()
+    source = (torch.randn(n, k, device="cuda") / 16).half()
+    bias, gamma, beta = torch.randn(n, device="cuda").half(), torch.rand(k, device="cuda").half(), torch.randn(k, device="cuda").half()
+    residual = torch.randn(*lead, n, device="cuda").half()
+    results = []
+    for o in (ops, slow):
+        if dtype == "int8":
+            w = o.upload_or_quantize_int8_weight(source, None, pkg.INT8WeightLoadOptions())
+            q = o.quantize_int8(x, 256)
+        elif dtype == "e4m3":
+            w = o.upload_fp8_weight(source, pkg.FP8WeightLoadOptions(scale_mode=pkg.FP8ScaleMode.PerOutputChannel))
+            quantised = o.quantize_e4m3(x)
+            q = (quantised.data, quantised.scales)
+        else:
+            w, q = o.fp16_weight(source), ()
+        out = [w.data, *([w.scales] if w.scales is not None else []), *q]
+        out += [o.linear(x, w), o.linear(x, w, bias, residual=residual), o.linear_activation(x, w, bias, pkg.ACT_GEGLU)]
+        calls = [pkg.LinearCall(x, w), pkg.LinearCall(x, w, bias, pkg.ACT_SILU)]
+        out += o.linear_grouped(calls)
+        assert calls[1].y is out[-1]
+        out.append(o.layer_norm(x, gamma, beta))
+        if dtype != "f16":
+            pair = o.layer_norm_quantized(x, gamma, beta, w)
+            out += [*pair, o.linear(None, w, bias, xq=pair[0], xq_scales=pair[1])]
+        results.append(out)
+    ctx.check()
+    for fast, plain in zip(*results):
+        assert fast.shape == plain.shape and fast.dtype == plain.dtype and torch.equal(fast, plain)
+
+
+def test_front_leaves_errors_to_the_python_path(gpu):
+    pkg, ctx, ops = gpu
+    w = ops.fp16_weight(torch.zeros(64, 32, device="cuda"))
+    with pytest.raises(pkg.CudaError, match="contiguous"):
+        ops.linear(torch.zeros(32, 8, device="cuda", dtype=torch.float16).t(), w)
+    with pytest.raises(pkg.CudaError, match="feature mismatch"):
+        ops.linear(torch.zeros(8, 16, device="cuda", dtype=torch.float16), w)
+    with pytest.raises(pkg.CudaError, match="requires a bias"):         # found by the library behind the front
+        ops.linear_activation(torch.zeros(8, 32, device="cuda", dtype=torch.float16), w, None, pkg.ACT_SILU)
