@@ -331,14 +331,25 @@ __device__ __forceinline__ void finish_chunk_16(const EpilogueTile& t, uint32_t 
                 out_words[i] = *reinterpret_cast<const uint32_t*>(&sum);
             }
         } else {
+            // The activation is chosen once per chunk, outside the loop over its values: the 16 evaluations of
+            // a lane are then independent chains that overlap (two epilogue warps per scheduler leave
+            // nothing else to hide an exp and a divide behind). With the choice and a branching divide per value a
+            // chunk took 1.2 us: QuickGELU of [154, 3072], FP16 K = 768, 10.7 us (7.3 without the arithmetic), now 8.1.
             float2 bias[8];
             read_staged<16>(t.column_bias, c0, bias);
+            if (t.activation == ACT_GELU) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float2 x = __fadd2_rn(from_half2_bits(out_words[i]), bias[i]);
-                out_words[i] = to_half2_bits(t.activation == ACT_GELU
-                                                 ? gelu_erf2(x)
-                                                 : make_float2(activate(x.x, t.activation), activate(x.y, t.activation)));
+                for (int i = 0; i < 8; ++i) {
+                    out_words[i] = to_half2_bits(gelu_erf2(__fadd2_rn(from_half2_bits(out_words[i]), bias[i])));
+                }
+            } else {
+                const float factor = t.activation == ACT_SILU ? -1.0f : -1.702f;    // SiLU, QuickGELU
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float2 x = __fadd2_rn(from_half2_bits(out_words[i]), bias[i]);
+                    out_words[i] = to_half2_bits(make_float2(divide_by_denominator(x.x, 1.0f + expf(factor * x.x)),
+                                                             divide_by_denominator(x.y, 1.0f + expf(factor * x.y))));
+                }
             }
         }
     }

@@ -219,6 +219,20 @@ __device__ __forceinline__ float2 gelu_erf2(float2 x) {
     return __fmul2_rn(__fmul2_rn(x, make_float2(0.5f, 0.5f)), one_plus_erf2(x));
 }
 
+// x / d for the denominators 1 + exp(..) of SiLU and QuickGELU (d >= 1, up to +inf), without a branch: the product
+// with the hardware reciprocal and one residual correction, q + (x - q d) r (Markstein, IBM J. Res. Dev. 34, 1990),
+// within one unit in the last place of the FP32 quotient, which is then rounded to FP16.
+// d is held below 2^126, where the reciprocal is still a normal number: the quotient of any larger d rounds
+// to an FP16 zero of x's sign either way. An infinite x has no finite residual and keeps the product.
+__device__ __forceinline__ float divide_by_denominator(float x, float d) {
+    d = fminf(d, 8.507059173023462e37f);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    const float q = x * r;
+    const float corrected = fmaf(fmaf(-q, d, x), r, q);
+    return fabsf(x) <= 3.402823466e+38f ? corrected : q;
+}
+
 // SiLU / GELU / QuickGELU on the FP32 value (ACT_NONE returns x).
 __device__ __forceinline__ float activate(float x, uint32_t activation) {
     if (activation == ACT_SILU) return x / (1.0f + expf(-x));

@@ -38,3 +38,47 @@ def test_residual_is_added_to_the_projection(gpu, dtype, pair, m, n, tile_n):
     assert torch.equal(in_place, want)
     assert amax.view(torch.float32).item() == want.abs().max().float().item()
     ctx.check()
+
+
+@pytest.mark.parametrize("name", ["silu", "gelu", "quick_gelu"])
+@pytest.mark.parametrize("n", [16, 40, 264])
+def test_activation_of_a_chunk(gpu, name, n):
+    """act(half(projection) + bias) against 64 bits from the same halves, over the whole FP16 range of arguments. The
+    FP32 evaluation is good to a few 2^-22 relative (2^-20 absolute for GELU's tail), so its FP16 rounding is at most
+    one step from the exactly rounded one."""
+    pkg, ctx, ops = gpu
+    k = 64
+    weight = ops.fp16_weight(torch.eye(n, k, device="cuda").half())
+    values = torch.cat([torch.linspace(-12, 12, 4000), torch.tensor([0.0, -0.0, 65504.0, -65504.0, 88.0, -88.0, 104.0, -104.0, 6e-8, -6e-8]),
+                        10.0 ** torch.linspace(-7, 4.8, 500), -(10.0 ** torch.linspace(-7, 4.8, 500))]).half()
+    columns = min(n, k)
+    m = -(-values.numel() // columns)
+    x = torch.zeros(m * columns).half()
+    x[:values.numel()] = values
+    padded = torch.zeros(m, k).half()
+    padded[:, :columns] = x.view(m, columns)
+    activation = {"silu": pkg.ACT_SILU, "gelu": pkg.ACT_GELU, "quick_gelu": pkg.ACT_QUICK_GELU}[name]
+    got = ops.linear_activation(padded.cuda(), weight, torch.zeros(n, device="cuda").half(), activation).cpu()
+    ctx.check()
+    z = torch.zeros(m, n, dtype=torch.float64)
+    z[:, :columns] = padded[:, :columns].double()
+    if name == "gelu":
+        from scipy.special import erfc
+        want = torch.from_numpy(0.5 * z.numpy() * erfc(-z.numpy() / np.sqrt(2.0)))
+    else:
+        want = z * torch.sigmoid(z * (1.0 if name == "silu" else 1.702))
+    rounded = want.half()
+    step = torch.maximum(rounded.double().abs() * 2.0 ** -10, torch.full_like(want, 2.0 ** -24))
+    assert (got.double() - rounded.double()).abs().le(step + 2.0 ** -20 * (name == "gelu")).all()
+
+
+def test_activation_of_infinities(gpu):
+    """x / (1 + exp(-x)) as IEEE has it: +inf stays, -inf and NaN give NaN."""
+    pkg, ctx, ops = gpu
+    weight = ops.fp16_weight(torch.eye(16, 64, device="cuda").half() * 2)
+    x = torch.zeros(3, 64).half()
+    x[0, 0], x[1, 0], x[2, 0] = 65504.0, -65504.0, float("nan")       # doubled: +-inf
+    for activation in (pkg.ACT_SILU, pkg.ACT_QUICK_GELU):
+        y = ops.linear_activation(x.cuda(), weight, torch.zeros(16, device="cuda").half(), activation).cpu()
+        assert y[0, 0] == float("inf") and torch.isnan(y[1, 0]) and torch.isnan(y[2]).all()
+    ctx.check()
