@@ -589,26 +589,28 @@ __device__ __forceinline__ bool issue_tile_mmas(MmaCursor& c, uint32_t tmem_d, u
     uint32_t stage = c.stage, phase = c.phase;
     uint32_t accumulate = 0;
     for (uint32_t kb = 0; kb < k_blocks; ++kb) {
-        if (!ptx::mbar_wait_bounded(c.full_base + stage * 8u, phase, c.abort_word, c.limit)) return false;
+        if (!ptx::warp_wait_bounded(c.full_base + stage * 8u, phase, c.abort_word, c.limit)) return false;
         ptx::tc_fence_after();
-        const uint32_t a_lo = c.a_lo_base + stage * c.stage_units;
-        if (c.mode == 0) {
-            ptx::umma_stage<KindTag, kPair>(tmem_d, a_lo, a_lo + c.b_units, ptx::kUmmaDescHiSw128, idesc, accumulate);
-        } else if (c.mode == 2 && KindTag != 0) {   // the one-MMA diagnostic exists for INT8 only
-            ptx::umma_stage<KindTag, kPair>(tmem_d, a_lo, a_lo + c.b_units, ptx::kUmmaDescHiSw128, idesc, accumulate);
-        } else if (c.mode == 2) {
-            const uint64_t hi = static_cast<uint64_t>(ptx::kUmmaDescHiSw128) << 32;
-            if (kPair) ptx::umma_i8_pair(tmem_d, hi | a_lo, hi | (a_lo + c.b_units), idesc, accumulate);
-            else ptx::umma_i8(tmem_d, hi | a_lo, hi | (a_lo + c.b_units), idesc, accumulate);
+        if (ptx::elect_one()) {
+            const uint32_t a_lo = c.a_lo_base + stage * c.stage_units;
+            if (c.mode == 0) {
+                ptx::umma_stage<KindTag, kPair>(tmem_d, a_lo, a_lo + c.b_units, ptx::kUmmaDescHiSw128, idesc, accumulate);
+            } else if (c.mode == 2 && KindTag != 0) {   // the one-MMA diagnostic exists for INT8 only
+                ptx::umma_stage<KindTag, kPair>(tmem_d, a_lo, a_lo + c.b_units, ptx::kUmmaDescHiSw128, idesc, accumulate);
+            } else if (c.mode == 2) {
+                const uint64_t hi = static_cast<uint64_t>(ptx::kUmmaDescHiSw128) << 32;
+                if (kPair) ptx::umma_i8_pair(tmem_d, hi | a_lo, hi | (a_lo + c.b_units), idesc, accumulate);
+                else ptx::umma_i8(tmem_d, hi | a_lo, hi | (a_lo + c.b_units), idesc, accumulate);
+            }
+            const uint32_t empty_bar = c.empty_base + stage * 8u;
+            if (kPair) {
+                ptx::umma_commit_pair(empty_bar);                                 // frees the leader's stage
+                ptx::umma_commit_pair(c.peer_empty_base + stage * 8u);            // and the peer's
+            } else {
+                ptx::umma_commit(empty_bar);
+            }
         }
         accumulate = 1;
-        const uint32_t empty_bar = c.empty_base + stage * 8u;
-        if (kPair) {
-            ptx::umma_commit_pair(empty_bar);                                 // frees the leader's stage
-            ptx::umma_commit_pair(c.peer_empty_base + stage * 8u);            // and the peer's
-        } else {
-            ptx::umma_commit(empty_bar);
-        }
         if (++stage == c.num_stages) { stage = 0; phase ^= 1u; }
     }
     c.stage = stage;
@@ -704,7 +706,8 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
     ptx::setmaxnreg_dec<kControlRegisters>();
     if (warp == 0) {
         // ------------------------------- TMA producer -------------------------------------
-        if (lane == 0) {
+        // like the MMA issuer below: the whole warp walks, one elected lane issues
+        {
             uint32_t stage = 0, phase = 0;
             uint32_t issued = 0;                     // stages handed to the copy engine so far
             const uint32_t full_base = ptx::smem_u32(&control->full[0]);
@@ -721,8 +724,10 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
                 const CUtensorMap* tmap_a = &problem->tmap_a;
                 const CUtensorMap* tmap_b = &problem->tmap_b;
                 if (params.problems != nullptr && problem != bound) {
-                    ptx::fence_tensormap_acquire(tmap_a);
-                    ptx::fence_tensormap_acquire(tmap_b);
+                    if (ptx::elect_one()) {
+                        ptx::fence_tensormap_acquire(tmap_a);
+                        ptx::fence_tensormap_acquire(tmap_b);
+                    }
                     bound = problem;
                 }
                 const bool geglu = work.activation == ACT_GEGLU;
@@ -741,7 +746,7 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
                 const uint32_t k_blocks = (skip_loads && skip_mma) ? 0u : work.k_blocks;
                 int32_t k0 = 0;
                 for (uint32_t kb = 0; kb < k_blocks; ++kb, k0 += k_step) {
-                    if (!ptx::mbar_wait_bounded(empty_base + stage * 8u, phase ^ 1u, abort_word, limit)) {
+                    if (!ptx::warp_wait_bounded(empty_base + stage * 8u, phase ^ 1u, abort_word, limit)) {
                         raise_abort(control, params.error_word, DEV_TIMEOUT_PRODUCER);
                         ok = false;
                         break;
@@ -749,20 +754,22 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
                     const uint32_t full_bar = full_base + stage * 8u;
                     const uint32_t a_dst = stages_base + stage * stage_bytes;
                     const uint32_t b_dst = a_dst + b_offset;
-                    if (skip_loads) {
-                        if (leader) ptx::mbar_arrive(full_bar);
-                    } else if (kPair) {
-                        if (leader) ptx::mbar_expect_tx(full_bar, tx_bytes);
-                        ptx::tma_load_2d_pair(a_dst, tmap_a, full_bar, k0, row_a);
-                        ptx::tma_load_2d_pair(b_dst, tmap_b, full_bar, k0, row_b_pair);
-                    } else if (a_loads_only) {      // diagnostic: half of the copy instructions, a third of the bytes
-                        ptx::mbar_expect_tx(full_bar, kTileM * kTileKBytes);
-                        ptx::tma_load_2d(a_dst, tmap_a, full_bar, k0, row_a);
-                    } else {
-                        ptx::mbar_expect_tx(full_bar, tx_bytes);
-                        ptx::tma_load_2d(a_dst, tmap_a, full_bar, k0, row_a);
-                        ptx::tma_load_2d(b_dst, tmap_b, full_bar, k0, row_b);
-                        if (geglu) ptx::tma_load_2d(b_dst + half * kTileKBytes, tmap_b, full_bar, k0, row_gate);
+                    if (ptx::elect_one()) {
+                        if (skip_loads) {
+                            if (leader) ptx::mbar_arrive(full_bar);
+                        } else if (kPair) {
+                            if (leader) ptx::mbar_expect_tx(full_bar, tx_bytes);
+                            ptx::tma_load_2d_pair(a_dst, tmap_a, full_bar, k0, row_a);
+                            ptx::tma_load_2d_pair(b_dst, tmap_b, full_bar, k0, row_b_pair);
+                        } else if (a_loads_only) {      // diagnostic: half of the copy instructions, a third of the bytes
+                            ptx::mbar_expect_tx(full_bar, kTileM * kTileKBytes);
+                            ptx::tma_load_2d(a_dst, tmap_a, full_bar, k0, row_a);
+                        } else {
+                            ptx::mbar_expect_tx(full_bar, tx_bytes);
+                            ptx::tma_load_2d(a_dst, tmap_a, full_bar, k0, row_a);
+                            ptx::tma_load_2d(b_dst, tmap_b, full_bar, k0, row_b);
+                            if (geglu) ptx::tma_load_2d(b_dst + half * kTileKBytes, tmap_b, full_bar, k0, row_gate);
+                        }
                     }
                     ++issued;
                     if (++stage == num_stages) { stage = 0; phase ^= 1u; }
@@ -780,10 +787,12 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
         }
     } else if (warp == 1) {
         // ------------------------------- MMA issuer ---------------------------------------
-        // One thread issues every MMA of the CTA (of the pair). Its loop is the critical path of
-        // the kernel: per stage it runs one barrier poll, one fence, one statement with the four
-        // MMAs and one commit, all on 32-bit values kept in registers.
-        if (lane == 0 && leader) {
+        // This loop is the critical path of the kernel: per stage one barrier poll, one fence, one statement with
+        // the four MMAs and one commit. The whole warp walks the tiles and one elected lane issues: the loop's
+        // values are then uniform to the compiler, while a loop run by one lane of a divergent warp issued a stage
+        // (four MMAs) per 0.3 us whatever its width. FP16 [2048, 1280], K = 5120: 35.4 -> 24.3 us (0.48 -> 0.69 of
+        // the measured tensor rate); FP8: 17.3 -> 14.8 us.
+        if (leader) {
             MmaCursor cursor;
             cursor.stage = 0;
             cursor.phase = 0;
@@ -814,7 +823,7 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
 #endif
                 for (uint32_t q = first_quarter; ok && q < first_quarter + quarters; ++q) {
                     // the quarter's previous user (if any) has been drained by every epilogue warp
-                    ok = ptx::mbar_wait_bounded(ptx::smem_u32(&control->acc_empty[q]), ((ring.parity >> q) & 1u) ^ 1u,
+                    ok = ptx::warp_wait_bounded(ptx::smem_u32(&control->acc_empty[q]), ((ring.parity >> q) & 1u) ^ 1u,
                                                 abort_word, limit);
                     ring.parity ^= 1u << q;
                 }
@@ -841,11 +850,13 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
                     break;
                 }
                 const uint32_t full_bar = ptx::smem_u32(&control->acc_full[first_quarter]);
-                if (kPair) {
-                    ptx::umma_commit_pair(full_bar);
-                    ptx::umma_commit_pair(ptx::map_to_cta(full_bar, 1));
-                } else {
-                    ptx::umma_commit(full_bar);
+                if (ptx::elect_one()) {                 // the lane that issued the MMAs
+                    if (kPair) {
+                        ptx::umma_commit_pair(full_bar);
+                        ptx::umma_commit_pair(ptx::map_to_cta(full_bar, 1));
+                    } else {
+                        ptx::umma_commit(full_bar);
+                    }
                 }
 #ifdef SDXLQ_DIAGNOSTICS
                 diag_issue += clock64() - diag_t_issue;

@@ -18,6 +18,19 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
 
+// True in one lane of the warp, the same one each time; all 32 lanes take part.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t elected;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(elected));
+    return elected != 0;
+}
+
 __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
@@ -65,6 +78,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
                                                   long long limit_cycles) {
     if (mbar_try_wait(bar, parity)) return true;
     return mbar_wait_slow(bar, parity, abort_word, limit_cycles);
+}
+
+// The same wait by all lanes of a warp, with one answer for the warp: true when every lane saw the phase complete.
+// (A lane that gave up alone would leave the others waiting for it in the next elect.sync.)
+__device__ __forceinline__ bool warp_wait_bounded(uint32_t bar, uint32_t parity, volatile uint32_t* abort_word,
+                                                  long long limit_cycles) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_word, limit_cycles));
 }
 
 // ---- TMA ---------------------------------------------------------------------------------
