@@ -44,8 +44,8 @@ def test_residual_is_added_to_the_projection(gpu, dtype, pair, m, n, tile_n):
 @pytest.mark.parametrize("n", [16, 40, 264])
 def test_activation_of_a_chunk(gpu, name, n):
     """act(half(projection) + bias) against 64 bits from the same halves, over the whole FP16 range of arguments. The
-    FP32 evaluation is good to a few 2^-22 relative (2^-20 absolute for GELU's tail), so its FP16 rounding is at most
-    one step from the exactly rounded one."""
+    FP32 evaluation is good to a few 2^-22 relative, and GELU's to |x| / 2 times the 6e-7 of its erfc, so its FP16 rounding
+    is within that and one step of the exactly rounded one."""
     pkg, ctx, ops = gpu
     k = 64
     weight = ops.fp16_weight(torch.eye(n, k, device="cuda").half())
@@ -69,7 +69,7 @@ def test_activation_of_a_chunk(gpu, name, n):
         want = z * torch.sigmoid(z * (1.0 if name == "silu" else 1.702))
     rounded = want.half()
     step = torch.maximum(rounded.double().abs() * 2.0 ** -10, torch.full_like(want, 2.0 ** -24))
-    assert (got.double() - rounded.double()).abs().le(step + 2.0 ** -20 * (name == "gelu")).all()
+    assert (got.double() - rounded.double()).abs().le(step + 3e-7 * z.abs() * (name == "gelu")).all()
 
 
 def test_activation_of_infinities(gpu):
