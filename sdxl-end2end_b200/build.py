@@ -12,7 +12,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIBRARY = os.path.join(HERE, "libsdxlq.so")
 FRONT = os.path.join(HERE, "_front.so")
 FRONT_SOURCES = ["torch_front.cpp", os.path.join("..", "..", "include", "sdxlq.h")]
-SOURCES = ["capi.cu", "gemm_umma.cu", "quantize.cu", "quantize_int8_fast.cu", "linear_small.cu", "layer_norm.cu", "harness_norm.cu"]
+SOURCES = ["capi.cu", "gemm_umma.cu", "quantize.cu", "quantize_int8_fast.cu", "linear_small.cu", "linear_skinny.cu", "layer_norm.cu", "harness_norm.cu"]
 HEADERS = ["internal.cuh", "ptx.cuh", "quantize.cuh", "fp8_math.cuh", "int8_math.cuh", os.path.join("..", "..", "include", "sdxlq.h")]
 
 NVCC_FLAGS = [

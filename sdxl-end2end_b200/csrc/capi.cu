@@ -29,6 +29,8 @@ cudaError_t launch_umma_gemm(const GemmLaunchParams& params, uint32_t grid, size
 size_t umma_gemm_control_bytes();
 cudaError_t launch_small_linear(const void* a, const void* b, const EpilogueParams& ep, uint32_t k_major,
                                 cudaStream_t stream);
+cudaError_t launch_skinny_linear(const void* a, const void* b, const EpilogueParams& ep, bool from_half, uint32_t sm_count,
+                                 cudaStream_t stream, bool early_launch);
 cudaError_t launch_bounded_wait_probe(uint32_t* error_word, long long limit_cycles, cudaStream_t stream);
 cudaError_t launch_int8_plain_rows(const QuantInt8Launch& launch, uint32_t blocks, uint32_t max_vectors,
                                    cudaStream_t stream, bool early_launch);
@@ -289,6 +291,14 @@ struct SmallCall {
     uint32_t k_major;
 };
 
+// A projection of few rows (linear_skinny.cu). `from_half`: `a` is the FP16 input, quantised by the kernel itself.
+struct SkinnyCall {
+    const void* a;
+    const void* b;
+    EpilogueParams ep;
+    bool from_half;
+};
+
 // INT8 quantiser jobs of one kernel flavour (one launch each).
 struct Int8JobSet {
     std::vector<QuantInt8Job> jobs;
@@ -308,6 +318,7 @@ struct Prepared {
     std::vector<TileRef> tiles[2];
     uint32_t max_cta_b_rows[2] = {0, 0};     // most B rows one CTA stages (tile_n, or tile_n / 2 in a pair)
     std::vector<SmallCall> small;
+    std::vector<SkinnyCall> skinny;
     uint32_t fp8_blocks = 0;
     uint32_t int8_linears = 0;
     uint32_t int8_small = 0;
@@ -482,6 +493,25 @@ void choose_quantiser_block(const sdxlq_context* ctx, Int8JobSet& set) {
     }
 }
 
+// Single projections of at most kSkinnyRows rows (one row tile of that kernel's MMA) take the kernel that splits K over
+// warps; figures at linear_skinny.cu. It loads operands 16 bytes at a time; a forced tile shape asks for the other kernel.
+constexpr uint64_t kSkinnyRows = 16;
+// Every block reads the whole FP16 input when it quantises for itself: up to 256 KB of it, and INT8 rows of the length
+// that the stand-alone quantiser takes.
+constexpr uint64_t kSkinnyInput = 131072, kSkinnyInt8Row = 16384;
+
+bool skinny_weight(const sdxlq_context* ctx, const sdxlq_linear_desc& d, size_t count, bool grouped) {
+    const sdxlq_weight& w = d.weight;
+    return !grouped && count == 1 && d.m <= kSkinnyRows && ctx->forced_tile_n == 0 && ctx->pair_mode == 0 && w.layout == SDXLQ_ROW_MAJOR_NK &&
+           w.k * (w.dtype == SDXLQ_FP16 ? 2u : 1u) % 16 == 0 && reinterpret_cast<uintptr_t>(w.data) % 16 == 0;
+}
+
+bool skinny_quantises(const sdxlq_linear_desc& d) {
+    const sdxlq_weight& w = d.weight;
+    return d.x_amax == nullptr && reinterpret_cast<uintptr_t>(d.x) % 16 == 0 && d.m * w.k <= kSkinnyInput &&
+           (w.dtype != SDXLQ_INT8 || (w.convrot_group_size == 0 && w.k <= kSkinnyInt8Row));
+}
+
 int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bool grouped, Prepared& prep) {
     std::map<QuantKey, std::pair<const void*, const float*>> shared_inputs;
     size_t scratch = 0;
@@ -496,6 +526,8 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
                               : w.dtype == SDXLQ_FP8_E5M2 ? KIND_E5M2 : KIND_F16;
         const void* a = d.x;
         const float* a_scales = nullptr;
+        const bool skinny = skinny_weight(ctx, d, count, grouped);
+        bool from_half = false;
         if (kind == KIND_I8 || kind == KIND_E4M3 || kind == KIND_E5M2) {
             if (d.xq != nullptr) {
                 a = d.xq;
@@ -515,7 +547,9 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
                     }
                     uint8_t* q = ctx->workspace + q_offset;
                     float* s = reinterpret_cast<float*>(ctx->workspace + s_offset);
-                    if (kind == KIND_I8) {
+                    if (skinny && skinny_quantises(d)) {
+                        from_half = true;                       // no quantiser launch
+                    } else if (kind == KIND_I8) {
                         const int job_status = add_int8_job(ctx, prep, d.x, false, d.m, w.k, w.convrot_group_size,
                                                             reinterpret_cast<int8_t*>(q), s, grouped);
                         if (job_status != SDXLQ_OK) return job_status;
@@ -528,8 +562,10 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
                     }
                     found = shared_inputs.emplace(key, std::make_pair(static_cast<const void*>(q), static_cast<const float*>(s))).first;
                 }
-                a = found->second.first;
-                a_scales = found->second.second;
+                if (!from_half) {
+                    a = found->second.first;
+                    a_scales = found->second.second;
+                }
             }
         }
 
@@ -559,6 +595,10 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
                             reinterpret_cast<uintptr_t>(a) % 16 == 0 &&
                             reinterpret_cast<uintptr_t>(w.data) % 16 == 0;
         if (kind == KIND_I8) ++prep.int8_linears;
+        if (skinny && reinterpret_cast<uintptr_t>(a) % 16 == 0) {
+            prep.skinny.push_back(SkinnyCall{a, w.data, ep, from_half});
+            continue;
+        }
         if (!tma_ok) {
             if (kind == KIND_I8) ++prep.int8_small;
             prep.small.push_back(SmallCall{a, w.data, ep, w.layout == SDXLQ_K_MAJOR_KN ? 1u : 0u});
@@ -847,6 +887,12 @@ int run_prepared(sdxlq_context* ctx, const Prepared& prep, const sdxlq_group_pla
     }
     status = run_small(ctx, prep);
     if (status != SDXLQ_OK) return status;
+    for (const SkinnyCall& call : prep.skinny) {
+        LaunchTimer timer(ctx, SDXLQ_KERNEL_GEMM);
+        const cudaError_t error = launch_skinny_linear(call.a, call.b, call.ep, call.from_half, static_cast<uint32_t>(ctx->sm_count),
+                                                       ctx->stream, ctx->early_launch && !ctx->profiling);
+        if (error != cudaSuccess) return fail_cuda(ctx, error, "few-row linear launch");
+    }
     count_stats(ctx, prep);
     return SDXLQ_OK;
 }

@@ -1,0 +1,88 @@
+"""Projections of at most 16 rows (csrc/linear_skinny.cu) against the tensor-memory GEMM, which a forced tile width
+brings back: INT8 bit-equal. FP8 and FP16 sum in another order: K / 16 MMA steps, each off by at most 2^-23 of a partial
+sum no larger than the sum S of the products' magnitudes, then the FP16 rounding of the projection may fall the other way."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def matrix(n, k):
+    return (torch.randn(n, k, device="cuda") / k ** 0.5).half()
+
+
+def make(pkg, ops, dtype, n, k, source):
+    if dtype.startswith("int8"):
+        group = int(dtype[4:] or 0)
+        return ops.upload_or_quantize_int8_weight(source, None, pkg.INT8WeightLoadOptions(enable_convrot=group != 0, convrot_group_size=group))
+    if dtype == "f16":
+        return ops.fp16_weight(source)
+    fmt = {"e4m3": pkg.ScalarType.Float8E4M3, "e5m2": pkg.ScalarType.Float8E5M2}[dtype]
+    mode = pkg.FP8ScaleMode.PerOutputChannel if k % 32 else pkg.FP8ScaleMode.TensorWide
+    return ops.upload_fp8_weight(source, pkg.FP8WeightLoadOptions(format=fmt, scale_mode=mode))
+
+
+def agree(got, want, exact, bound):
+    if exact:
+        assert torch.equal(got, want)
+    else:
+        assert ((got.float() - want.float()).abs() <= bound + want.abs().float() * 2.0 ** -10).all()
+
+
+@pytest.mark.parametrize("dtype", ["int8", "int864", "int8256", "e4m3", "e5m2", "f16"])
+@pytest.mark.parametrize("m,n,k", [(1, 16, 256), (2, 1280, 320), (7, 24, 1040), (8, 2600, 64), (9, 5200, 512), (16, 1280, 2816), (16, 40, 5120), (13, 8, 16)])
+def test_against_the_tensor_memory_gemm(gpu, dtype, m, n, k):
+    pkg, ctx, ops = gpu
+    if dtype.startswith("int8") and k % int(dtype[4:] or 1):
+        pytest.skip("the group size does not divide K")
+    torch.manual_seed(n + k)
+    source = matrix(n, k)
+    weight = make(pkg, ops, dtype, n, k, source)
+    x = torch.randn(m, k, device="cuda").half()
+    x[:, :: max(1, k // 3)] *= 20
+    bias, residual = torch.randn(n, device="cuda").half(), torch.randn(m, n, device="cuda").half()
+    amax = torch.zeros(2, dtype=torch.int32, device="cuda")
+    results = []
+    for tile in (0, 32):
+        ctx.set_tile_n(tile)
+        out = [ops.linear(x, weight), ops.linear(x, weight, bias, residual=residual, y_amax=amax[tile // 32:][:1])]
+        out += [ops.linear_activation(x, weight, bias, a) for a in (pkg.ACT_SILU, pkg.ACT_GELU, pkg.ACT_QUICK_GELU, pkg.ACT_GEGLU)]
+        if dtype.startswith("int8"):
+            accumulators = torch.zeros(m, n, dtype=torch.int32, device="cuda")
+            ops.linear(x, weight, acc_out=accumulators)
+            out.append(accumulators)
+        results.append(out)
+    ctx.set_tile_n(0)
+    ctx.check()
+    projection = results[1][0].abs().float()
+    magnitudes = 1.2 * x.abs().float() @ source.abs().float().T          # 1.2: quantised values are up to an eighth larger
+    off = projection * 2.0 ** -10 + k / 16 * 2.0 ** -23 * magnitudes     # of the projection
+    half = n // 2
+    value, gate = projection[:, :half] + 5.0, projection[:, half:] + 5.0     # with their bias
+    bounds = [off, off] + [1.2 * off] * 3 + [off[:, :half] * gate + 1.2 * value * off[:, half:]]      # activations' slope: < 1.2
+    for at, (got, want) in enumerate(zip(*results)):
+        # INT8: the FP16 result of the exp-based activations may differ by the last step of the two quotients
+        agree(got, want, dtype.startswith("int8") and at not in (2, 4), bounds[at] if at < 6 else None)
+    assert amax[:1].view(torch.float32).item() == results[0][1].abs().max().float().item()
+
+
+@pytest.mark.parametrize("dtype", ["int8", "e4m3", "e5m2"])
+@pytest.mark.parametrize("m,k", [(1, 64), (2, 1280), (16, 2816), (16, 8208)])
+def test_own_quantisation_is_the_quantisers(gpu, dtype, m, k):
+    """FP16 input and input cast by the stand-alone quantiser give the same bits (also past the size at which the kernel
+    quantises for itself), for rows of zeros, infinities (INT8: the finite maximum) and tiny values too."""
+    pkg, ctx, ops = gpu
+    torch.manual_seed(k)
+    weight = make(pkg, ops, dtype, 96, k, matrix(96, k))
+    x = torch.randn(m, k, device="cuda").half()
+    if m > 2:
+        x[1], x[2] = 0.0, x[2] * 1e-7
+        if dtype == "int8":
+            x[3, 5] = float("inf")
+    if dtype == "int8":
+        xq, scales = ops.quantize_int8(x, 0)
+    else:
+        quantised = ops.quantize_fp8(x, weight.type)
+        xq, scales = quantised.data, quantised.scales
+    assert torch.equal(ops.linear(x, weight), ops.linear(None, weight, xq=xq, xq_scales=scales))
+    ctx.check()
