@@ -1405,7 +1405,8 @@ int sdxlq_pack_weight_fp8(sdxlq_context* ctx, const void* src, int32_t src_dtype
     }
     const cudaError_t error = launch_fp8_weight_pack(src, src_dtype, static_cast<uint32_t>(n), static_cast<uint32_t>(k),
                                                      fmt == SDXLQ_FP8_E4M3 ? 0 : 1, per_channel,
-                                                     layout == SDXLQ_K_MAJOR_KN ? 1 : 0, dst, scales, ctx->stream);
+                                                     layout == SDXLQ_K_MAJOR_KN ? 1 : 0, dst, scales, ctx->stream,
+                                                     ctx->early_launch && !ctx->profiling);
     if (error != cudaSuccess) return fail_cuda(ctx, error, "FP8 weight pack launch");
     return SDXLQ_OK;
 }

@@ -509,9 +509,85 @@ __global__ void fill_f32_kernel(float* values, uint32_t count, float value) {
     if (index < count) values[index] = value;
 }
 
+// Row-major weights with a scale per output channel in one launch: a block reads its row once with 16-byte loads,
+// holds it from the maximum to the cast (rows of up to 5120 values; what is longer is read again) and writes eight
+// bytes at a time. Same arithmetic as the three kernels above, which walk the matrix twice value by value behind a
+// memset and stay for tensor-wide scales, FP8 sources, K-major layouts and unaligned rows. Packing a
+// 1280-wide transformer block (52 M values, ten calls): FP16 258 -> 71 us, FP32 268 -> 77 us.
+constexpr int kPackHeld = 5;
+constexpr uint32_t kPackThreads = 128;
+
+template <typename In>
+__global__ void __launch_bounds__(kPackThreads)
+fp8_weight_rows_kernel(const In* source, uint32_t k, uint32_t fmt, uint8_t* destination, float* scales) {
+    __shared__ float warp_maximum[kPackThreads / 32];
+    wait_for_prior_kernels_then_release_next();
+    const uint32_t vectors = k / 8;
+    const In* row = source + static_cast<size_t>(blockIdx.x) * k;
+    float held[kPackHeld][8];
+    float local = 0.0f;
+    const auto widest = [&](const float (&values)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float magnitude = fabsf(values[i]);
+            if (magnitude <= 3.402823466e+38f && magnitude > local) local = magnitude;      // finite only
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < kPackHeld; ++u) {
+        const uint32_t vector = threadIdx.x + u * kPackThreads;
+        load8(row + vector * 8u, vector < vectors, vector < vectors ? 8u : 0u, held[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < kPackHeld; ++u) widest(held[u]);
+    for (uint32_t vector = threadIdx.x + kPackHeld * kPackThreads; vector < vectors; vector += kPackThreads) {
+        float values[8];
+        load8(row + vector * 8u, true, 8u, values);
+        widest(values);
+    }
+#pragma unroll
+    for (int offset = 16; offset > 0; offset >>= 1) local = fmaxf(local, __shfl_xor_sync(0xffffffffu, local, offset));
+    if ((threadIdx.x & 31u) == 0) warp_maximum[threadIdx.x >> 5] = local;
+    __syncthreads();
+#pragma unroll
+    for (uint32_t w = 0; w < kPackThreads / 32; ++w) local = fmaxf(local, warp_maximum[w]);
+    const float scale = fp8_scale_from_amax(local, fmt);
+    if (threadIdx.x == 0) scales[blockIdx.x] = scale;
+    uint2* packed = reinterpret_cast<uint2*>(destination + static_cast<size_t>(blockIdx.x) * k);
+    const auto cast = [&](const float (&values)[8]) {
+        uint32_t words[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t lo = encode_fp8x2(__fdiv_rn(values[4 * i], scale), __fdiv_rn(values[4 * i + 1], scale), fmt);
+            const uint32_t hi = encode_fp8x2(__fdiv_rn(values[4 * i + 2], scale), __fdiv_rn(values[4 * i + 3], scale), fmt);
+            words[i] = (lo & 0xFFFFu) | (hi << 16);
+        }
+        return make_uint2(words[0], words[1]);
+    };
+#pragma unroll
+    for (int u = 0; u < kPackHeld; ++u) {
+        const uint32_t vector = threadIdx.x + u * kPackThreads;
+        if (vector < vectors) packed[vector] = cast(held[u]);
+    }
+    for (uint32_t vector = threadIdx.x + kPackHeld * kPackThreads; vector < vectors; vector += kPackThreads) {
+        float values[8];
+        load8(row + vector * 8u, true, 8u, values);
+        packed[vector] = cast(values);
+    }
+}
+
 cudaError_t launch_fp8_weight_pack(const void* source, int32_t dtype, uint32_t n, uint32_t k, uint32_t fmt,
                                    uint32_t per_channel, uint32_t k_major, uint8_t* destination,
-                                   float* scales, cudaStream_t stream) {
+                                   float* scales, cudaStream_t stream, bool early_launch) {
+    if (per_channel != 0 && k_major == 0 && (dtype == 3 || dtype == 4) && k % 8 == 0 && reinterpret_cast<uintptr_t>(source) % 16 == 0 &&
+        reinterpret_cast<uintptr_t>(destination) % 8 == 0) {
+        if (dtype == 3) {
+            return launch_behind(fp8_weight_rows_kernel<__half>, n, kPackThreads, 0, stream, early_launch, static_cast<const __half*>(source),
+                                 k, fmt, destination, scales);
+        }
+        return launch_behind(fp8_weight_rows_kernel<float>, n, kPackThreads, 0, stream, early_launch, static_cast<const float*>(source), k, fmt,
+                             destination, scales);
+    }
     const uint32_t scale_count = per_channel ? n : 1;
     cudaError_t status = cudaMemsetAsync(scales, 0, scale_count * sizeof(float), stream);
     if (status != cudaSuccess) return status;

@@ -96,7 +96,7 @@ cudaError_t launch_fp8_quantize(const QuantFp8Launch& launch, uint32_t blocks, c
                                 bool skip_maximum_pass);
 cudaError_t launch_fp8_weight_pack(const void* source, int32_t dtype, uint32_t n, uint32_t k, uint32_t fmt,
                                    uint32_t per_channel, uint32_t k_major, uint8_t* destination,
-                                   float* scales, cudaStream_t stream);
+                                   float* scales, cudaStream_t stream, bool early_launch);
 cudaError_t launch_fill_f32(float* values, uint32_t count, float value, cudaStream_t stream);
 
 // LayerNorm over the last dimension of FP16 x[rows, width] (width a multiple of 8, at most 2048, 16-byte
