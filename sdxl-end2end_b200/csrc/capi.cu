@@ -60,6 +60,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 
 size_t align_up(size_t value, size_t alignment) { return (value + alignment - 1) / alignment * alignment; }
 
+constexpr int kPairChosen = 2;
+
 }  // namespace
 
 struct sdxlq_context {
@@ -77,8 +79,8 @@ struct sdxlq_context {
     int geglu_tile_n = 0;                     // tuning: accumulator tile width of GEGLU projections in grouped launches
                                               // (0: cost model). 128 lets the MMA issuer run three tiles ahead of the
                                               // GEGLU epilogues but measured slower (operand traffic, per-tile costs).
-    int pair_mode = 0;                        // 0 never use CTA pairs (default: they measured no faster), 1 whenever
-                                              // possible, -1 for traffic-bound launches only
+    int pair_mode = kPairChosen;              // kPairChosen: where they measured faster (see choose_tile); 0 never use
+                                              // CTA pairs, 1 whenever possible, -1 for traffic-bound launches only
     uint32_t diagnostic_skip = 0;             // SDXLQ_DIAGNOSTIC_SKIP: tuning aid, see GemmLaunchParams
     long long wait_limit_cycles = 4000000000LL;
     int forced_tile_n = 0;
@@ -222,7 +224,7 @@ struct TileChoice {
     bool pair;
 };
 
-TileChoice choose_tile(const sdxlq_context* ctx, uint32_t m, uint32_t n, bool geglu, bool grouped, uint32_t siblings = 1) {
+TileChoice choose_tile(const sdxlq_context* ctx, uint32_t m, uint32_t n, uint32_t k_blocks, bool geglu, bool grouped, uint32_t siblings = 1) {
     const uint32_t step = geglu ? 32 : 16;
     const uint32_t tiles_m = (m + kTileM - 1) / kTileM;
     const uint32_t sms = static_cast<uint32_t>(ctx->sm_count);
@@ -230,8 +232,17 @@ TileChoice choose_tile(const sdxlq_context* ctx, uint32_t m, uint32_t n, bool ge
     // `siblings`: problems of (about) this shape that share the launch (a small inline group)
     const uint64_t tiles_at_widest = static_cast<uint64_t>(siblings) * tiles_m * ((columns + (geglu ? 127 : 255)) / (geglu ? 128 : 256));
     const bool traffic_bound = grouped ? tiles_m >= 2 : tiles_at_widest >= 3ull * sms;
-    // CTA pairs are opt-in (pair_mode): single calls, inline groups and plans all take them then.
-    const bool pair_allowed = ctx->pair_mode != 0 && m > kTileM && (traffic_bound || ctx->pair_mode == 1);
+    // CTA pairs halve the weight bytes per SM. Chosen for GEGLU launches of many tiles, and in launches of few for a K of
+    // at least 32 stages, or 20 from 4096 rows on (us, single CTAs against pairs, FP8 | FP16): GEGLU [2048, 10240],
+    // K = 1280: 26.6, 24.0 | 43.6, 39.6; [8192, 5120], K = 640: 37.0, 34.2 | 46.3, 41.3; [140, 1280], K = 5120: 11.4, 10.9 |
+    // 21.2, 19.1; [2048, 1280], K = 5120: 14.6, 13.8 | 23.9, 21.6; [8192, 640], K = 2560: 15.7, 14.7 | 25.6, 23.1. Not
+    // for shorter K (FP16 [1000, 1280], K = 1280, 20 stages: 11.7, 11.8, its q/k/v 11.6, 12.5), not for launches of many
+    // tiles without GEGLU (FP16 [65536, 640], K = 640: 79, 91), and not in plans, whose tiles would be split over two
+    // launches. set_pair_mode makes it never, always or by traffic.
+    bool pair_allowed = ctx->pair_mode != 0 && m > kTileM && (traffic_bound || ctx->pair_mode == 1);
+    if (ctx->pair_mode == kPairChosen) {
+        pair_allowed = !grouped && ctx->forced_tile_n == 0 && m > kTileM && (geglu ? traffic_bound : !traffic_bound && k_blocks >= (m < 4096 ? 32u : 20u));
+    }
     if (ctx->forced_tile_n >= 16) {
         const uint32_t forced = std::min<uint32_t>(kMaxTileN, static_cast<uint32_t>(ctx->forced_tile_n));
         const uint32_t pair_step = 32;
@@ -250,11 +261,12 @@ TileChoice choose_tile(const sdxlq_context* ctx, uint32_t m, uint32_t n, bool ge
             const uint32_t per_tile = geglu ? tile_n / 2 : tile_n;
             const uint32_t tiles_n = (columns + per_tile - 1) / per_tile;
             double cost;
-            if (traffic_bound || pair) {
+            if (traffic_bound || (pair && ctx->pair_mode != kPairChosen)) {
                 cost = static_cast<double>(tiles_n) * (128.0 + (pair ? tile_n / 2.0 : tile_n));
             } else {
-                const uint64_t tiles = static_cast<uint64_t>(siblings) * tiles_m * tiles_n;
-                const uint64_t waves = (tiles + sms - 1) / sms;
+                const uint64_t workers = pair ? sms / 2 : sms;
+                const uint64_t tiles = static_cast<uint64_t>(siblings) * (pair ? (tiles_m + 1) / 2 : tiles_m) * tiles_n;
+                const uint64_t waves = (tiles + workers - 1) / workers;
                 cost = static_cast<double>(waves) * (tile_n + 32.0);
             }
             if (cost < best_cost) { best_cost = cost; best = TileChoice{tile_n, pair != 0}; }
@@ -505,7 +517,7 @@ constexpr uint64_t kSkinnyInput = 131072, kSkinnyInt8Row = 16384;
 
 bool skinny_weight(const sdxlq_context* ctx, const sdxlq_linear_desc& d, size_t count, bool grouped) {
     const sdxlq_weight& w = d.weight;
-    return !grouped && count == 1 && d.m <= kSkinnyRows && ctx->forced_tile_n == 0 && ctx->pair_mode == 0 && w.layout == SDXLQ_ROW_MAJOR_NK &&
+    return !grouped && count == 1 && d.m <= kSkinnyRows && ctx->forced_tile_n == 0 && ctx->pair_mode != 1 && ctx->pair_mode != -1 && w.layout == SDXLQ_ROW_MAJOR_NK &&
            w.k * (w.dtype == SDXLQ_FP16 ? 2u : 1u) % 16 == 0 && reinterpret_cast<uintptr_t>(w.data) % 16 == 0;
 }
 
@@ -610,14 +622,15 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
 
         GemmProblem problem{};
         problem.ep = ep;
-        const TileChoice choice = choose_tile(ctx, ep.m, ep.n, geglu, grouped, grouped ? 1u : static_cast<uint32_t>(count));
+        const uint32_t k_blocks = static_cast<uint32_t>((w.k * element + kTileKBytes - 1) / kTileKBytes);
+        const TileChoice choice = choose_tile(ctx, ep.m, ep.n, k_blocks, geglu, grouped, grouped ? 1u : static_cast<uint32_t>(count));
         const int flavour = choice.pair ? 1 : 0;
         const uint32_t rows_per_tile = choice.pair ? 2 * kTileM : kTileM;
         problem.tile_n = choice.tile_n;
         const uint32_t per_tile = geglu ? problem.tile_n / 2 : problem.tile_n;
         problem.tiles_m = (ep.m + rows_per_tile - 1) / rows_per_tile;
         problem.tiles_n = (ep.n_out + per_tile - 1) / per_tile;
-        problem.k_blocks = static_cast<uint32_t>((w.k * element + kTileKBytes - 1) / kTileKBytes);
+        problem.k_blocks = k_blocks;
         const uint32_t format = kind == KIND_I8 ? 1u : (kind == KIND_E5M2 ? 1u : 0u);
         // c_format: 2 = S32 for kind::i8, 1 = F32 otherwise; operands K-major; M = 128 (256 for a pair).
         problem.idesc = ((kind == KIND_I8 ? 2u : 1u) << 4) | (format << 7) | (format << 10) |

@@ -1,0 +1,39 @@
+"""Shapes for which single calls take CTA pairs by themselves (GEGLU of many tiles, a long K with few), at and beside
+the rule's edges: INT8 results equal those of single CTAs bit for bit, FP8 and FP16 too (the MMAs of a pair add the same
+products in the same order)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", ["int8", "e4m3", "f16"])
+@pytest.mark.parametrize("m,n,k,geglu", [(129, 64, 4096, False), (154, 1280, 5120, False), (257, 648, 4112, False), (2048, 1280, 3968, False), (4097, 640, 2560, False),
+                                         (1976, 1280, 5120, False), (128, 1280, 5120, False), (3000, 5120, 640, True), (8192, 5120, 128, True),
+                                         (1976, 10240, 1280, True)])
+def test_same_bits_as_single_ctas(pkg, gpu_session, dtype, m, n, k, geglu):
+    _, _, reference = gpu_session
+    reference.ctx.set_pair_mode(0)
+    reference.ctx.set_tile_n(0)
+    context = pkg.Context(0, workspace_bytes=256 << 20)
+    ops = pkg.Ops(context, poison_outputs=True)
+    torch.manual_seed(m)
+    source = (torch.randn(n, k, device="cuda") / k ** 0.5).half()
+    if dtype == "int8":
+        weight = ops.upload_or_quantize_int8_weight(source, None, pkg.INT8WeightLoadOptions(enable_convrot=False))
+    elif dtype == "e4m3":
+        weight = ops.upload_fp8_weight(source, pkg.FP8WeightLoadOptions(scale_mode=pkg.FP8ScaleMode.PerOutputChannel))
+    else:
+        weight = ops.fp16_weight(source)
+    x, bias = torch.randn(m, k, device="cuda").half(), torch.randn(n, device="cuda").half()
+    for o in (ops, reference):
+        if geglu:
+            o.result = [o.linear_activation(x, weight, bias, pkg.ACT_GEGLU)]
+        else:
+            residual = torch.randn(m, n, device="cuda", generator=torch.Generator("cuda").manual_seed(1)).half()
+            o.result = [o.linear(x, weight, bias), o.linear(x, weight, bias, residual=residual)]
+            o.result += o.linear_grouped([pkg.LinearCall(x, weight), pkg.LinearCall(x, weight, bias)])
+    context.check()
+    for got, want in zip(ops.result, reference.result):
+        assert torch.equal(got, want)
+    context.close()
