@@ -600,7 +600,7 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
         ep.kind = kind;
         ep.activation = static_cast<uint32_t>(d.activation);
         ep.w_scale_per_channel = (kind != KIND_F16 && w.scale_count != 1) ? 1 : 0;
-        ep.vector_store_ok = (reinterpret_cast<uintptr_t>(d.y) % 16 == 0) && (ep.n_out % 8 == 0);
+        ep.vector_store_ok = row_access_ok(ep, 16);
         ep.vector_meta_ok = (reinterpret_cast<uintptr_t>(w.scales) % 16 == 0) &&
                             (reinterpret_cast<uintptr_t>(d.bias) % 16 == 0) &&
                             (!geglu || ep.n_out % 8 == 0);

@@ -41,9 +41,15 @@ struct EpilogueParams {
     uint32_t kind;               // GemmKind
     uint32_t activation;         // Activation
     uint32_t w_scale_per_channel;
-    uint32_t vector_store_ok;    // y rows are 16-byte aligned and n_out % 8 == 0
+    uint32_t vector_store_ok;    // row_access_ok(.., 16)
     uint32_t vector_meta_ok;     // w_scales / bias (and their GEGLU gate halves) are 16-byte aligned
 };
+
+// Whether the rows of y, and of the residual that is loaded the same way, take accesses of `bytes` bytes. The residual
+// has its own alignment: it need not alias y.
+__host__ __device__ inline bool row_access_ok(const EpilogueParams& ep, uint32_t bytes) {
+    return reinterpret_cast<uintptr_t>(ep.y) % bytes == 0 && reinterpret_cast<uintptr_t>(ep.residual) % bytes == 0 && ep.n_out % (bytes / 2) == 0;
+}
 
 // One GEMM problem of a grouped launch. Tensor maps first (64-byte alignment required).
 struct alignas(64) GemmProblem {
@@ -64,8 +70,8 @@ struct alignas(64) GemmProblem {
 enum TileFlags : uint16_t {
     TILE_HAS_BIAS = 1,          // bias != null
     TILE_SCALE_PER_CHANNEL = 2, // w_scales has one entry per weight row (else one entry)
-    TILE_STORE_16 = 4,          // y rows 16-byte aligned and n_out % 8 == 0
-    TILE_STORE_32 = 8,          // y rows 32-byte aligned and n_out % 16 == 0
+    TILE_STORE_16 = 4,          // rows of y and the residual 16-byte aligned
+    TILE_STORE_32 = 8,          // rows of y and the residual 32-byte aligned
     TILE_RAW_ACCUMULATORS = 16, // the problem also wants its INT32 accumulators (ep.acc_out)
     TILE_HAS_RESIDUAL = 32,     // ep.residual is added after the bias (no activation)
     TILE_OUTPUT_AMAX = 64,      // ep.y_amax receives the maximum of |y|
@@ -104,7 +110,7 @@ __host__ __device__ inline TileRef make_tile_ref(const GemmProblem& problem, uin
     r.tile_n = static_cast<uint16_t>(problem.tile_n);
     r.kind = static_cast<uint8_t>(ep.kind);
     r.activation = static_cast<uint8_t>(ep.activation);
-    const bool store_32 = ep.vector_store_ok != 0 && ep.n_out % 16 == 0 && reinterpret_cast<uintptr_t>(ep.y) % 32 == 0;
+    const bool store_32 = row_access_ok(ep, 32);
     r.flags = static_cast<uint16_t>((ep.bias != nullptr ? TILE_HAS_BIAS : 0) |
                                     (ep.kind != KIND_F16 && ep.w_scale_per_channel != 0 ? TILE_SCALE_PER_CHANNEL : 0) |
                                     (ep.vector_store_ok != 0 ? TILE_STORE_16 : 0) | (store_32 ? TILE_STORE_32 : 0) |

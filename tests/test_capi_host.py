@@ -86,6 +86,34 @@ def test_cxx_shim_compiles_against_the_header(tmp_path):
     assert subprocess.run([str(tmp_path / "shim")]).returncode == 0
 
 
+def test_row_accesses_follow_the_residual_too(pkg, tmp_path):
+    """The epilogue loads a residual as wide as it stores y: 16 or 32 bytes only where both are aligned for it."""
+    source = tmp_path / "rows.cu"
+    source.write_text(
+        '#include "internal.cuh"\n#include <cstdio>\n#include <cstdlib>\n'
+        "int main(int, char** v) {\n"
+        "  sdxlq::GemmProblem p{};\n"
+        "  p.ep.y = reinterpret_cast<__half*>(4096 + std::atoi(v[1]));\n"
+        "  if (std::atoi(v[2]) >= 0) p.ep.residual = reinterpret_cast<__half*>(8192 + std::atoi(v[2]));\n"
+        "  p.ep.n = p.ep.n_out = std::atoi(v[3]);\n"
+        "  p.ep.vector_store_ok = sdxlq::row_access_ok(p.ep, 16);\n"
+        "  const unsigned flags = sdxlq::make_tile_ref(p, 0, 0, 0).flags;\n"
+        '  std::printf("%d", (flags & sdxlq::TILE_STORE_32) ? 32 : (flags & sdxlq::TILE_STORE_16) ? 16 : 2);\n'
+        "}\n")
+    binary = tmp_path / "rows"
+    subprocess.run([os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"), "-std=c++20", "-gencode", "arch=compute_100a,code=sm_100a",
+                    "-I", pkg.api._build.CSRC, str(source), "-o", str(binary)], check=True)
+
+    def widest(y, residual, columns):
+        return int(subprocess.run([str(binary), str(y), str(residual), str(columns)], capture_output=True, check=True).stdout)
+
+    for y in (0, 2, 16, 32):
+        for residual in (-1, 0, 2, 8, 16, 48, 64):
+            for columns in (16, 24, 17):
+                at = [y, 2 * columns] + ([residual] if residual >= 0 else [])
+                assert widest(y, residual, columns) == next(w for w in (32, 16, 2) if all(v % w == 0 for v in at))
+
+
 def test_enum_values_match_the_reference(pkg):
     # include/sdxl/cuda/tensor.hpp:17-48 and ops.hpp:15 of the reference
     assert [int(v) for v in pkg.ScalarType] == [0, 1, 2, 3, 4, 5]

@@ -40,6 +40,20 @@ def test_residual_is_added_to_the_projection(gpu, dtype, pair, m, n, tile_n):
     ctx.check()
 
 
+@pytest.mark.parametrize("offset", [1, 8, 24])
+@pytest.mark.parametrize("m", [3, 130])
+def test_residual_with_an_alignment_of_its_own(gpu, offset, m):
+    """A contiguous residual 2, 16 or 48 bytes into its buffer, beside an output that takes 32-byte accesses."""
+    pkg, ctx, ops = gpu
+    torch.manual_seed(offset)
+    n, k = 48, 64
+    weight = packed(pkg, ops, "f16", n, k)
+    x, bias = torch.randn(m, k, device="cuda").half(), torch.randn(n, device="cuda").half()
+    residual = torch.randn(m * n + offset, device="cuda").half()[offset:].view(m, n)
+    assert torch.equal(ops.linear(x, weight, bias, residual=residual), ops.linear(x, weight, bias) + residual)
+    ctx.check()
+
+
 @pytest.mark.parametrize("name", ["silu", "gelu", "quick_gelu"])
 @pytest.mark.parametrize("n", [16, 40, 264])
 def test_activation_of_a_chunk(gpu, name, n):
