@@ -226,17 +226,19 @@ __device__ __forceinline__ float2 gelu_erf2(float2 x) {
 }
 
 // x / d for the denominators 1 + exp(..) of SiLU and QuickGELU (d >= 1, up to +inf), without a branch: the product
-// with the hardware reciprocal and one residual correction, q + (x - q d) r (Markstein, IBM J. Res. Dev. 34, 1990),
-// within one unit in the last place of the FP32 quotient, which is then rounded to FP16.
-// d is held below 2^126, where the reciprocal is still a normal number: the quotient of any larger d rounds
-// to an FP16 zero of x's sign either way. An infinite x has no finite residual and keeps the product.
+// with the hardware reciprocal and one residual correction, q - (q d - x) r (Markstein, IBM J. Res. Dev. 34, 1990).
+// d is clamped to 2^126, where the reciprocal is still a normal number: the quotient of any larger d rounds to an
+// FP16 zero of x's sign either way. The residual is q d - x and not x - q d, whose +0 would turn the quotient of
+// -0 into +0. An infinite x has no residual: +inf keeps the product; -inf (over d = +inf) takes the NaN of its residual,
+// which is what the division gives. Rounded to FP16 the result equals that of the division for every x that is a sum of two
+// FP16 values (all 2^32 of them compared on the GPU, both factors).
 __device__ __forceinline__ float divide_by_denominator(float x, float d) {
     d = fminf(d, 8.507059173023462e37f);
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     const float q = x * r;
-    const float corrected = fmaf(fmaf(-q, d, x), r, q);
-    return fabsf(x) <= 3.402823466e+38f ? corrected : q;
+    const float corrected = fmaf(-fmaf(q, d, -x), r, q);
+    return x <= 3.402823466e+38f ? corrected : q;
 }
 
 // SiLU / GELU / QuickGELU on the FP32 value (ACT_NONE returns x).

@@ -86,13 +86,24 @@ def test_activation_of_a_chunk(gpu, name, n):
     assert (got.double() - rounded.double()).abs().le(step + 3e-7 * z.abs() * (name == "gelu")).all()
 
 
-def test_activation_of_infinities(gpu):
-    """x / (1 + exp(-x)) as IEEE has it: +inf stays, -inf and NaN give NaN."""
+@pytest.mark.parametrize("m,tile_n", [(3, 0), (3, 16), (17, 0), (130, 0)])
+def test_activation_of_infinities_and_zeros(gpu, m, tile_n):
+    """x / (1 + exp(-x)) as IEEE has it: +inf stays, -inf and NaN give NaN, a zero keeps its sign; on the few-row
+    kernel (3 rows) and in the epilogue of the tensor-memory GEMM (a forced tile width, or more than 16 rows)."""
     pkg, ctx, ops = gpu
-    weight = ops.fp16_weight(torch.eye(16, 64, device="cuda").half() * 2)
-    x = torch.zeros(3, 64).half()
-    x[0, 0], x[1, 0], x[2, 0] = 65504.0, -65504.0, float("nan")       # doubled: +-inf
+    ctx.set_tile_n(tile_n)
+    weight = torch.eye(16, 64, device="cuda").half() * 2
+    weight[1, 1] = 0.25
+    weight = ops.fp16_weight(weight)
+    bias = torch.zeros(16, device="cuda").half()
+    bias[1] = -0.0
+    x = torch.zeros(m, 64).half()
+    last = m - 1
+    x[last - 2, 0], x[last - 1, 0], x[last, 0] = 65504.0, -65504.0, float("nan")       # doubled: +-inf
+    x[last - 2, 1] = -2.0 ** -24                                                      # a quarter of it rounds to -0
     for activation in (pkg.ACT_SILU, pkg.ACT_QUICK_GELU):
-        y = ops.linear_activation(x.cuda(), weight, torch.zeros(16, device="cuda").half(), activation).cpu()
-        assert y[0, 0] == float("inf") and torch.isnan(y[1, 0]) and torch.isnan(y[2]).all()
+        y = ops.linear_activation(x.cuda(), weight, bias, activation).cpu()
+        assert y[last - 2, 0] == float("inf") and torch.isnan(y[last - 1, 0]) and torch.isnan(y[last]).all()
+        assert y[last - 2, 1] == 0 and torch.signbit(y[last - 2, 1]) and not torch.signbit(y[last - 2, 2])
+    ctx.set_tile_n(0)
     ctx.check()
