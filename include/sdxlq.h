@@ -88,7 +88,8 @@ typedef struct sdxlq_linear_desc {
     const void* bias;            /* FP16 [N] or NULL */
     int32_t activation;          /* sdxlq_activation; anything but NONE requires bias */
     int32_t reserved0;
-    void* y;                     /* FP16 [M,N]; [M,N/2] for GEGLU */
+    void* y;                     /* FP16 [M,N]; [M,N/2] for GEGLU. May overlap x where the call quantises it (INT8 and
+                                  * FP8 weights without xq) */
     /* Optional reuse of already quantised activations (the three attention projections share
      * one input; the cross-attention K/V projections share the text context). When xq is set,
      * x is not read. INT8: xq INT8 [M,K] rotated with the weight's group size, xq_scales [M].

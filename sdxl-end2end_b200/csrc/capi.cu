@@ -515,15 +515,30 @@ constexpr uint64_t kSkinnyRows = 16;
 // that the stand-alone quantiser takes.
 constexpr uint64_t kSkinnyInput = 131072, kSkinnyInt8Row = 16384;
 
-bool skinny_weight(const sdxlq_context* ctx, const sdxlq_linear_desc& d, size_t count, bool grouped) {
+bool overlap(const void* a, uint64_t a_bytes, const void* b, uint64_t b_bytes) {
+    const uintptr_t first = reinterpret_cast<uintptr_t>(a), second = reinterpret_cast<uintptr_t>(b);
+    return a != nullptr && b != nullptr && first < second + b_bytes && second < first + a_bytes;
+}
+
+// Its blocks read all of their activations while others already write, so these have to be apart from the outputs. A
+// square projection in place is quantised by the launch in front instead, which has read x before the first store.
+bool outputs_apart(const sdxlq_linear_desc& d, const void* input, uint64_t input_bytes) {
+    const uint64_t n_out = d.activation == SDXLQ_ACT_GEGLU ? d.weight.n / 2 : d.weight.n;
+    return !overlap(input, input_bytes, d.y, d.m * n_out * 2) && !overlap(input, input_bytes, d.acc_out, d.m * d.weight.n * 4);
+}
+
+bool skinny_call(const sdxlq_context* ctx, const sdxlq_linear_desc& d, size_t count, bool grouped) {
     const sdxlq_weight& w = d.weight;
     return !grouped && count == 1 && d.m <= kSkinnyRows && ctx->forced_tile_n == 0 && ctx->pair_mode != 1 && ctx->pair_mode != -1 && w.layout == SDXLQ_ROW_MAJOR_NK &&
-           w.k * (w.dtype == SDXLQ_FP16 ? 2u : 1u) % 16 == 0 && reinterpret_cast<uintptr_t>(w.data) % 16 == 0;
+           w.k * (w.dtype == SDXLQ_FP16 ? 2u : 1u) % 16 == 0 && reinterpret_cast<uintptr_t>(w.data) % 16 == 0 &&
+           (w.dtype != SDXLQ_FP16 || outputs_apart(d, d.x, d.m * w.k * 2)) &&
+           (w.dtype == SDXLQ_FP16 || d.xq == nullptr || outputs_apart(d, d.xq, d.m * w.k));
 }
 
 bool skinny_quantises(const sdxlq_linear_desc& d) {
     const sdxlq_weight& w = d.weight;
     return d.x_amax == nullptr && reinterpret_cast<uintptr_t>(d.x) % 16 == 0 && d.m * w.k <= kSkinnyInput &&
+           outputs_apart(d, d.x, d.m * w.k * 2) &&
            (w.dtype != SDXLQ_INT8 || (w.convrot_group_size == 0 && w.k <= kSkinnyInt8Row));
 }
 
@@ -541,7 +556,7 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
                               : w.dtype == SDXLQ_FP8_E5M2 ? KIND_E5M2 : KIND_F16;
         const void* a = d.x;
         const float* a_scales = nullptr;
-        const bool skinny = skinny_weight(ctx, d, count, grouped);
+        const bool skinny = skinny_call(ctx, d, count, grouped);
         bool from_half = false;
         if (kind == KIND_I8 || kind == KIND_E4M3 || kind == KIND_E5M2) {
             if (d.xq != nullptr) {

@@ -86,3 +86,24 @@ def test_own_quantisation_is_the_quantisers(gpu, dtype, m, k):
         xq, scales = quantised.data, quantised.scales
     assert torch.equal(ops.linear(x, weight), ops.linear(None, weight, xq=xq, xq_scales=scales))
     ctx.check()
+
+
+@pytest.mark.parametrize("dtype", ["int8", "int8256", "e4m3", "e5m2"])
+@pytest.mark.parametrize("m,k,shift", [(2, 64, 0), (16, 1280, 0), (16, 1280, 640), (16, 5120, 0)])
+def test_projection_in_place(gpu, dtype, m, k, shift):
+    """A square projection written over its own input (or half a row behind it): the input is read whole before the first
+    store, also where the grid takes more than one wave of blocks ([16, 5120])."""
+    pkg, ctx, ops = gpu
+    if dtype == "int8256" and k % 256:
+        pytest.skip("the group size does not divide K")
+    torch.manual_seed(k)
+    weight = make(pkg, ops, dtype, k, k, matrix(k, k))
+    bias, values = torch.randn(k, device="cuda").half(), torch.randn(m, k, device="cuda").half()
+    want = ops.linear(values, weight, bias, residual=values)
+    for with_residual in (False, True) if shift == 0 else (False,):
+        buffer = torch.zeros(m * k + shift, device="cuda", dtype=torch.float16)
+        x, out = buffer[:m * k].view(m, k), buffer[shift:].view(m, k)
+        x.copy_(values)
+        ops.linear(x, weight, bias, residual=x if with_residual else None, out=out)
+        assert torch.equal(out, want if with_residual else ops.linear(values, weight, bias))
+    ctx.check()
