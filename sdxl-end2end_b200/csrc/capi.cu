@@ -224,7 +224,8 @@ struct TileChoice {
     bool pair;
 };
 
-TileChoice choose_tile(const sdxlq_context* ctx, uint32_t m, uint32_t n, uint32_t k_blocks, bool geglu, bool grouped, uint32_t siblings = 1) {
+TileChoice choose_tile(const sdxlq_context* ctx, uint32_t m, uint32_t n, uint32_t k_blocks, bool geglu, bool grouped, uint32_t siblings,
+                       bool allow_chosen_pairs) {
     const uint32_t step = geglu ? 32 : 16;
     const uint32_t tiles_m = (m + kTileM - 1) / kTileM;
     const uint32_t sms = static_cast<uint32_t>(ctx->sm_count);
@@ -241,7 +242,7 @@ TileChoice choose_tile(const sdxlq_context* ctx, uint32_t m, uint32_t n, uint32_
     // launches. set_pair_mode makes it never, always or by traffic.
     bool pair_allowed = ctx->pair_mode != 0 && m > kTileM && (traffic_bound || ctx->pair_mode == 1);
     if (ctx->pair_mode == kPairChosen) {
-        pair_allowed = !grouped && ctx->forced_tile_n == 0 && m > kTileM && (geglu ? traffic_bound : !traffic_bound && k_blocks >= (m < 4096 ? 32u : 20u));
+        pair_allowed = allow_chosen_pairs && !grouped && ctx->forced_tile_n == 0 && m > kTileM && (geglu ? traffic_bound : !traffic_bound && k_blocks >= (m < 4096 ? 32u : 20u));
     }
     if (ctx->forced_tile_n >= 16) {
         const uint32_t forced = std::min<uint32_t>(kMaxTileN, static_cast<uint32_t>(ctx->forced_tile_n));
@@ -301,6 +302,14 @@ struct SmallCall {
     const void* b;
     EpilogueParams ep;
     uint32_t k_major;
+};
+
+// A projection for the tensor-memory GEMM, before its tile shape is chosen.
+struct GemmCall {
+    EpilogueParams ep;
+    const void* a;
+    const void* b;
+    uint32_t k_blocks;
 };
 
 // A projection of few rows (linear_skinny.cu). `from_half`: `a` is the FP16 input, quantised by the kernel itself.
@@ -544,6 +553,7 @@ bool skinny_quantises(const sdxlq_linear_desc& d) {
 
 int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bool grouped, Prepared& prep) {
     std::map<QuantKey, std::pair<const void*, const float*>> shared_inputs;
+    std::vector<GemmCall> gemms;
     size_t scratch = 0;
     for (size_t index = 0; index < count; ++index) {
         const sdxlq_linear_desc& d = descs[index];
@@ -635,26 +645,42 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
             continue;
         }
 
+        gemms.push_back(GemmCall{ep, a, w.data, static_cast<uint32_t>((w.k * element + kTileKBytes - 1) / kTileKBytes)});
+    }
+
+    // A small group takes CTA pairs when every member would: split over the two flavours it would be two launches, which
+    // cost more than pairs give (us, one launch of single CTAs against both: FP16 [154, 1280], K = 1280 and [154, 1280],
+    // K = 2048: 9.6, 16.2; INT8 [300, 1280], K = 1280 and K = 5120: 11.3, 15.6).
+    const uint32_t siblings = grouped ? 1u : static_cast<uint32_t>(count);
+    const auto tile_for = [&](const GemmCall& call, bool allow_chosen_pairs) {
+        return choose_tile(ctx, call.ep.m, call.ep.n, call.k_blocks, call.ep.activation == ACT_GEGLU, grouped, siblings, allow_chosen_pairs);
+    };
+    bool allow_chosen_pairs = true;
+    if (!grouped && gemms.size() > 1) {
+        for (const GemmCall& call : gemms) allow_chosen_pairs = allow_chosen_pairs && tile_for(call, true).pair;
+    }
+    for (const GemmCall& call : gemms) {
+        const EpilogueParams& ep = call.ep;
+        const bool geglu = ep.activation == ACT_GEGLU;
         GemmProblem problem{};
         problem.ep = ep;
-        const uint32_t k_blocks = static_cast<uint32_t>((w.k * element + kTileKBytes - 1) / kTileKBytes);
-        const TileChoice choice = choose_tile(ctx, ep.m, ep.n, k_blocks, geglu, grouped, grouped ? 1u : static_cast<uint32_t>(count));
+        const TileChoice choice = tile_for(call, allow_chosen_pairs);
         const int flavour = choice.pair ? 1 : 0;
         const uint32_t rows_per_tile = choice.pair ? 2 * kTileM : kTileM;
         problem.tile_n = choice.tile_n;
         const uint32_t per_tile = geglu ? problem.tile_n / 2 : problem.tile_n;
         problem.tiles_m = (ep.m + rows_per_tile - 1) / rows_per_tile;
         problem.tiles_n = (ep.n_out + per_tile - 1) / per_tile;
-        problem.k_blocks = k_blocks;
-        const uint32_t format = kind == KIND_I8 ? 1u : (kind == KIND_E5M2 ? 1u : 0u);
+        problem.k_blocks = call.k_blocks;
+        const uint32_t format = ep.kind == KIND_I8 ? 1u : (ep.kind == KIND_E5M2 ? 1u : 0u);
         // c_format: 2 = S32 for kind::i8, 1 = F32 otherwise; operands K-major; M = 128 (256 for a pair).
-        problem.idesc = ((kind == KIND_I8 ? 2u : 1u) << 4) | (format << 7) | (format << 10) |
+        problem.idesc = ((ep.kind == KIND_I8 ? 2u : 1u) << 4) | (format << 7) | (format << 10) |
                         ((problem.tile_n >> 3) << 17) | ((rows_per_tile >> 4) << 24);
         // B box: the rows one TMA load brings in. A single CTA loads the whole tile (two boxes of
         // half the tile for GEGLU); each CTA of a pair loads half of the tile's rows.
         const uint32_t b_box_rows = choice.pair ? problem.tile_n / 2 : per_tile;
-        if (!encode_operand(ctx, &problem.tmap_a, kind, a, ep.m, w.k, kTileM) ||
-            !encode_operand(ctx, &problem.tmap_b, kind, w.data, w.n, w.k, b_box_rows)) {
+        if (!encode_operand(ctx, &problem.tmap_a, ep.kind, call.a, ep.m, ep.k, kTileM) ||
+            !encode_operand(ctx, &problem.tmap_b, ep.kind, call.b, ep.n, ep.k, b_box_rows)) {
             return fail(ctx, SDXLQ_ERR_CUDA, "cuTensorMapEncodeTiled rejected an operand");
         }
         prep.max_cta_b_rows[flavour] = std::max(prep.max_cta_b_rows[flavour], choice.pair ? problem.tile_n / 2 : problem.tile_n);

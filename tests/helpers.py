@@ -76,3 +76,20 @@ def reference_dense(oracle, x_f16: np.ndarray, w_f16: np.ndarray, bias_f16, acti
     if activation == 2:
         return (np.float32(0.5) * y * (np.float32(1.0) + erf(y * np.float32(0.7071067811865475)))).astype(np.float32)
     return (y / (np.float32(1.0) + np.exp(np.float32(-1.702) * y))).astype(np.float32)
+
+
+def launches(call) -> list:
+    """(name, blocks) of the CUDA kernels that `call` launches."""
+    import json
+    import tempfile
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as trace:
+        call()
+        torch.cuda.synchronize()
+    with tempfile.NamedTemporaryFile(suffix=".json") as file:
+        trace.export_chrome_trace(file.name)
+        events = json.load(open(file.name))["traceEvents"]
+    kernels = sorted((e for e in events if e.get("cat") == "kernel"), key=lambda e: e["ts"])
+    return [(e["name"], e["args"]["grid"][0]) for e in kernels]

@@ -4,7 +4,17 @@ products in the same order)."""
 import pytest
 import torch
 
+import helpers
+
 pytestmark = pytest.mark.gpu
+
+
+def pack(pkg, ops, dtype, source):
+    if dtype == "int8":
+        return ops.upload_or_quantize_int8_weight(source, None, pkg.INT8WeightLoadOptions(enable_convrot=False))
+    if dtype == "e4m3":
+        return ops.upload_fp8_weight(source, pkg.FP8WeightLoadOptions(scale_mode=pkg.FP8ScaleMode.PerOutputChannel))
+    return ops.fp16_weight(source)
 
 
 @pytest.mark.parametrize("dtype", ["int8", "e4m3", "f16"])
@@ -18,13 +28,7 @@ def test_same_bits_as_single_ctas(pkg, gpu_session, dtype, m, n, k, geglu):
     context = pkg.Context(0, workspace_bytes=256 << 20)
     ops = pkg.Ops(context, poison_outputs=True)
     torch.manual_seed(m)
-    source = (torch.randn(n, k, device="cuda") / k ** 0.5).half()
-    if dtype == "int8":
-        weight = ops.upload_or_quantize_int8_weight(source, None, pkg.INT8WeightLoadOptions(enable_convrot=False))
-    elif dtype == "e4m3":
-        weight = ops.upload_fp8_weight(source, pkg.FP8WeightLoadOptions(scale_mode=pkg.FP8ScaleMode.PerOutputChannel))
-    else:
-        weight = ops.fp16_weight(source)
+    weight = pack(pkg, ops, dtype, (torch.randn(n, k, device="cuda") / k ** 0.5).half())
     x, bias = torch.randn(m, k, device="cuda").half(), torch.randn(n, device="cuda").half()
     for o in (ops, reference):
         if geglu:
@@ -36,4 +40,33 @@ def test_same_bits_as_single_ctas(pkg, gpu_session, dtype, m, n, k, geglu):
     context.check()
     for got, want in zip(ops.result, reference.result):
         assert torch.equal(got, want)
+    context.close()
+
+
+@pytest.mark.parametrize("dtype", ["int8", "e4m3", "f16"])
+@pytest.mark.parametrize("shapes", [[(154, 1280, 1280), (154, 1280, 4096)], [(2048, 1280, 1280), (154, 1280, 4096), (154, 1280, 4096)],
+                                    [(300, 1280, 5120), (300, 1280, 64)], [(257, 648, 5120), (300, 1280, 5120)]])
+def test_a_small_group_is_one_launch(pkg, gpu_session, dtype, shapes):
+    """Members with and without pairs by the rule (a long K beside a short one), or all with pairs: one GEMM launch, and
+    the bits of the single calls."""
+    context = pkg.Context(0, workspace_bytes=256 << 20)
+    ops = pkg.Ops(context, poison_outputs=True)
+    torch.manual_seed(1)
+    calls = []
+    for m, n, k in shapes:
+        weight = pack(pkg, ops, dtype, (torch.randn(n, k, device="cuda") / k ** 0.5).half())
+        x = torch.randn(m, k, device="cuda").half()
+        given = {}
+        if dtype == "int8":
+            given = dict(zip(("xq", "xq_scales"), ops.quantize_int8(x, 0)))
+        elif dtype == "e4m3":
+            cast = ops.quantize_e4m3(x)
+            given = {"xq": cast.data, "xq_scales": cast.scales}
+        calls.append((x, weight, given))
+    grouped = []
+    names = helpers.launches(lambda: grouped.extend(ops.linear_grouped([pkg.LinearCall(x, w, **given) for x, w, given in calls])))
+    assert sum("sdxlq_umma_gemm_kernel" in name for name, _ in names) == 1
+    for got, (x, weight, given) in zip(grouped, calls):
+        assert torch.equal(got, ops.linear(x, weight, **given))
+    context.check()
     context.close()
