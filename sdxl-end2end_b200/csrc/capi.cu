@@ -458,7 +458,7 @@ int int8_quantiser_launches(const Prepared& prep) {
 }
 
 void add_fp8_job(Prepared& prep, const void* x, uint64_t count, uint32_t fmt, uint8_t* q, float* scale_out,
-                 bool grouped, uint32_t* amax_in = nullptr) {
+                 uint32_t* amax_in = nullptr) {
     QuantFp8Job job{};
     job.amax_in = amax_in;
     job.x = x;
@@ -467,14 +467,33 @@ void add_fp8_job(Prepared& prep, const void* x, uint64_t count, uint32_t fmt, ui
     job.count = count;
     job.fmt = fmt;
     job.vector_ok = (reinterpret_cast<uintptr_t>(x) % 16 == 0) && (reinterpret_cast<uintptr_t>(q) % 8 == 0);
-    job.first_block = prep.fp8_blocks;
-    // Grouped launches: 32768 values per block (four rounds of loads; with one round the job look-up, the reduction and the
-    // atomics of a block are as long as its loads: 743 projections in E5M2, maximum 1095 -> 1010 us, cast 1210 -> 1010 us).
-    const uint64_t per_block = grouped ? 32768 : 8192;
-    const uint64_t wanted = (count + per_block - 1) / per_block;
-    job.num_blocks = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(1184, wanted)));
-    prep.fp8_blocks += job.num_blocks;
     prep.fp8_jobs.push_back(job);
+}
+
+// Values that a block of the FP8 quantiser loads in one round: four 16-byte loads a thread.
+constexpr uint64_t kFp8Round = 8192;
+
+// Rounds per block of a grouped launch: as many as leave four blocks per SM, at most four. With few values the launch wants
+// every SM: K/V plan with one [154, 2048] input 12.7 us (maximum and cast) with one round, 14.9 with four; sixteen images
+// [2464, 2048] 16.6, 18.1. With many, the job look-up, the reduction and the atomics of a block are as long as one round of
+// loads: five inputs, 14 M values 18.5 us with one round, 15.9 with two; 29 M values 29.1, 22.9 with four; 743 projections at
+// 1024 x 1024 1791, 1503 (two), 1440 (three), 1412 (four).
+uint64_t fp8_values_per_block(const sdxlq_context* ctx, const Prepared& prep) {
+    uint64_t total = 0;
+    for (const QuantFp8Job& job : prep.fp8_jobs) total += job.count;
+    const uint64_t rounds = total / (kFp8Round * 4 * static_cast<uint64_t>(ctx->sm_count));
+    return kFp8Round * std::max<uint64_t>(1, std::min<uint64_t>(4, rounds));
+}
+
+// Lays the FP8 jobs of a launch out in blocks of `values_per_block` values, at most 1184 blocks a job.
+void lay_out_fp8_jobs(Prepared& prep, uint64_t values_per_block) {
+    prep.fp8_blocks = 0;
+    for (QuantFp8Job& job : prep.fp8_jobs) {
+        job.first_block = prep.fp8_blocks;
+        const uint64_t wanted = (job.count + values_per_block - 1) / values_per_block;
+        job.num_blocks = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(1184, wanted)));
+        prep.fp8_blocks += job.num_blocks;
+    }
 }
 
 void order_tiles(const sdxlq_context* ctx, const std::vector<GemmProblem>& problems, std::vector<TileRef>& tiles,
@@ -598,7 +617,7 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
                             return fail(ctx, SDXLQ_ERR_UNSUPPORTED_SHAPE, "too many distinct FP8 inputs in one grouped call");
                         }
                         add_fp8_job(prep, d.x, static_cast<uint64_t>(d.m) * w.k, kind == KIND_E4M3 ? 0 : 1, q, s,
-                                    grouped, static_cast<uint32_t*>(const_cast<void*>(d.x_amax)));
+                                    static_cast<uint32_t*>(const_cast<void*>(d.x_amax)));
                     }
                     found = shared_inputs.emplace(key, std::make_pair(static_cast<const void*>(q), static_cast<const float*>(s))).first;
                 }
@@ -699,6 +718,7 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
         if (!grouped || prep.problems[flavour].size() <= 1) continue;
         order_tiles(ctx, prep.problems[flavour], prep.tiles[flavour], flavour == 1);
     }
+    lay_out_fp8_jobs(prep, grouped ? fp8_values_per_block(ctx, prep) : kFp8Round);
     if (grouped) {
         choose_quantiser_block(ctx, prep.int8[INT8_GENERIC]);
         choose_quantiser_block(ctx, prep.int8[INT8_ROTATED]);
@@ -1257,7 +1277,8 @@ int sdxlq_quantize_act_fp8(sdxlq_context* ctx, const void* x_f16, uint64_t count
         return fail(ctx, SDXLQ_ERR_INVALID_ARGUMENT, "FP8 activation quantization requires float16 input and an FP8 destination");
     }
     Prepared prep;
-    add_fp8_job(prep, x_f16, count, fmt == SDXLQ_FP8_E4M3 ? 0 : 1, q, scale, false);
+    add_fp8_job(prep, x_f16, count, fmt == SDXLQ_FP8_E4M3 ? 0 : 1, q, scale);
+    lay_out_fp8_jobs(prep, kFp8Round);
     const QuantFp8Launch launch = bind_fp8(ctx, prep.fp8_jobs, nullptr);
     LaunchTimer timer(ctx, SDXLQ_KERNEL_QUANT_FP8, 2);
     const cudaError_t error = launch_fp8_quantize(launch, prep.fp8_blocks, ctx->stream, ctx->early_launch && !ctx->profiling, false);

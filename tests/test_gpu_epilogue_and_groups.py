@@ -336,3 +336,22 @@ def test_output_maximum_hand_over_to_the_fp8_quantiser(gpu, fmt, m, n, k, activa
         ctx.check()
         assert int(word.item()) == 0
         assert torch.equal(out, plain_out)
+
+
+@pytest.mark.parametrize("rows,inputs,rounds", [(154, 1, 1), (154, 6, 1), (2200, 1, 1), (2403, 2, 2), (4099, 2, 3), (4100, 5, 4)])
+def test_fp8_quantiser_blocks_follow_the_launch(gpu, rows, inputs, rounds):
+    """A plan's quantiser launches hold four blocks per SM before a block takes more than one round of 8192 values."""
+    pkg, ctx, ops = gpu
+    torch.manual_seed(rows)
+    k = 2048
+    weight = ops.upload_fp8_weight((torch.randn(64, k, device="cuda") / k ** 0.5).half(), pkg.FP8WeightLoadOptions())
+    xs = [torch.randn(rows, k, device="cuda").half() for _ in range(inputs)]
+    plan = ops.plan([pkg.LinearCall(x, weight) for x in xs])
+    names = H.launches(plan.run)
+    properties = torch.cuda.get_device_properties(0)
+    assert max(1, min(4, rows * k * inputs // (4 * 8192 * properties.multi_processor_count))) == rounds
+    blocks = [grid for name, grid in names if "fp8_amax" in name or "fp8_cast" in name]
+    assert blocks == [inputs * -(-rows * k // (8192 * rounds))] * 2
+    for call, x in zip(plan.calls, xs):
+        assert torch.equal(call.y, ops.linear(x, weight))
+    ctx.check()
