@@ -78,18 +78,32 @@ def reference_dense(oracle, x_f16: np.ndarray, w_f16: np.ndarray, bias_f16, acti
     return (y / (np.float32(1.0) + np.exp(np.float32(-1.702) * y))).astype(np.float32)
 
 
-def launches(call) -> list:
-    """(name, blocks) of the CUDA kernels that `call` launches."""
-    import json
-    import tempfile
+def launches(context, call) -> list:
+    """The kernels (name, blocks, cluster width) that `call` launches, read from a captured graph; nothing runs."""
+    from collections import namedtuple
     import torch
-    from torch.profiler import ProfilerActivity, profile
+    from cuda.bindings import driver
+
+    def checked(answer):
+        assert answer[0] == driver.CUresult.CUDA_SUCCESS, answer
+        return answer[1:] if len(answer) != 2 else answer[1]
+
+    Kernel = namedtuple("Kernel", "name blocks cluster")
+    call()                                                  # what happens once per process is done before the capture
     torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as trace:
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
+    context.set_stream(stream)
+    with torch.cuda.graph(graph, stream=stream):
         call()
-        torch.cuda.synchronize()
-    with tempfile.NamedTemporaryFile(suffix=".json") as file:
-        trace.export_chrome_trace(file.name)
-        events = json.load(open(file.name))["traceEvents"]
-    kernels = sorted((e for e in events if e.get("cat") == "kernel"), key=lambda e: e["ts"])
-    return [(e["name"], e["args"]["grid"][0]) for e in kernels]
+    context.set_stream(torch.cuda.current_stream())
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    count = checked(driver.cuGraphGetNodes(raw))[1]
+    kernels = []
+    for node in checked(driver.cuGraphGetNodes(raw, count))[0][:count]:
+        if checked(driver.cuGraphNodeGetType(node)) != driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            continue
+        params = checked(driver.cuGraphKernelNodeGetParams(node))
+        name = checked(driver.cuFuncGetName(params.func) if int(params.func) else driver.cuKernelGetName(params.kern)).decode()
+        shape = checked(driver.cuGraphKernelNodeGetAttribute(node, driver.CUkernelNodeAttrID.CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION))
+        kernels.append(Kernel(name, params.gridDimX, max(1, shape.clusterDim.x)))
+    return kernels

@@ -347,11 +347,12 @@ def test_fp8_quantiser_blocks_follow_the_launch(gpu, rows, inputs, rounds):
     weight = ops.upload_fp8_weight((torch.randn(64, k, device="cuda") / k ** 0.5).half(), pkg.FP8WeightLoadOptions())
     xs = [torch.randn(rows, k, device="cuda").half() for _ in range(inputs)]
     plan = ops.plan([pkg.LinearCall(x, weight) for x in xs])
-    names = H.launches(plan.run)
+    kernels = H.launches(ctx, plan.run)
     properties = torch.cuda.get_device_properties(0)
     assert max(1, min(4, rows * k * inputs // (4 * 8192 * properties.multi_processor_count))) == rounds
-    blocks = [grid for name, grid in names if "fp8_amax" in name or "fp8_cast" in name]
+    blocks = [kernel.blocks for kernel in kernels if "fp8_amax" in kernel.name or "fp8_cast" in kernel.name]
     assert blocks == [inputs * -(-rows * k // (8192 * rounds))] * 2
+    plan.run()
     for call, x in zip(plan.calls, xs):
         assert torch.equal(call.y, ops.linear(x, weight))
     ctx.check()
