@@ -79,7 +79,7 @@ struct sdxlq_context {
     int geglu_tile_n = 0;                     // tuning: accumulator tile width of GEGLU projections in grouped launches
                                               // (0: cost model). 128 lets the MMA issuer run three tiles ahead of the
                                               // GEGLU epilogues but measured slower (operand traffic, per-tile costs).
-    int pair_mode = kPairChosen;              // kPairChosen: where they measured faster (see choose_tile); 0 never use
+    int pair_mode = kPairChosen;              // kPairChosen: where they measured faster (see pairs_pay); 0 never use
                                               // CTA pairs, 1 whenever possible, -1 for traffic-bound launches only
     uint32_t diagnostic_skip = 0;             // SDXLQ_DIAGNOSTIC_SKIP: tuning aid, see GemmLaunchParams
     long long wait_limit_cycles = 4000000000LL;
@@ -218,64 +218,81 @@ int validate(sdxlq_context* ctx, const sdxlq_linear_desc& d) {
 //    bound by operand traffic into shared memory. A single CTA moves (128 + t) bytes per k-byte for
 //    128 * t MACs; a CTA pair moves (256 + t) for 256 * t. Cost of a projection per 128 rows:
 //    ceil(N / t) * (128 + t), or ceil(N / t) * (128 + t / 2) for a pair (last-tile padding included).
-//  * A launch of few tiles is bound by how many SMs get work: single CTAs, minimise waves * (t + 32).
+//  * A launch of few tiles is bound by how many SMs (pairs of SMs) get work: minimise waves * (t + 32).
 struct TileChoice {
     uint32_t tile_n;
     bool pair;
 };
 
-TileChoice choose_tile(const sdxlq_context* ctx, uint32_t m, uint32_t n, uint32_t k_blocks, bool geglu, bool grouped, uint32_t siblings,
+// Whether a call or small group that left the choice to the library takes CTA pairs; `waves` and `tile_n` are those of its
+// single CTAs. A pair halves the weight bytes per SM, which pays in GEGLU launches of many tiles, and in launches of few
+// tiles for a long K (us, single CTAs against pairs, FP8 | FP16 | INT8): GEGLU [2048, 10240], K = 1280: 27.1, 24.7 |
+// 47.8, 42.9 | 27.7, 25.0; [8192, 5120], K = 640: 36.3, 33.5 | 47.3, 42.9 | 38.1, 35.5; [140, 1280], K = 5120: 12.1, 11.7 |
+// 23.2, 21.5 | 11.0, 10.5; [2048, 1280], K = 5120: 14.3, 13.8 | 24.4, 22.3 | 14.0, 13.6; [8192, 640], K = 2560: 16.1,
+// 15.1 | 26.0, 23.7 | 15.8, 14.8. Where the single CTAs are one wave a pair has no second tile to gain on and a later start:
+// there it wants 32 stages of K, and 64 beside tiles of 224 columns and more ([6000, 640], K = 2560, 224 wide: 18.1, 18.7 |
+// 17.3, 17.4 | 12.0, 12.4; [3000, 1280], K = 5120, 224 wide: 17.5, 17.5 | 33.9, 31.1 | 16.6, 16.8; [2560, 1280], K = 5120, 192
+// wide: 15.6, 15.4 | 27.4, 26.5 | 15.2, 15.1). Not for shorter K (FP16 [1000, 1280], K = 1280, 20 stages: 11.7, 11.8), not
+// for launches of many tiles without GEGLU (FP16 [65536, 640], K = 640: 79, 91), and not in plans, whose tiles would be
+// split over two launches.
+bool pairs_pay(uint32_t m, uint32_t k_blocks, bool geglu, bool many_tiles, uint64_t waves, uint32_t tile_n) {
+    if (m <= kTileM || geglu != many_tiles) return false;
+    if (geglu) return true;
+    if (waves > 1) return k_blocks >= (m < 4096 ? 32u : 20u);
+    return k_blocks >= (tile_n < 224 ? 32u : 64u);
+}
+
+TileChoice choose_tile(const sdxlq_context* ctx, const EpilogueParams& ep, uint32_t k_blocks, bool grouped, uint32_t siblings,
                        bool allow_chosen_pairs) {
+    const bool geglu = ep.activation == ACT_GEGLU;
     const uint32_t step = geglu ? 32 : 16;
-    const uint32_t tiles_m = (m + kTileM - 1) / kTileM;
+    const uint32_t tiles_m = (ep.m + kTileM - 1) / kTileM;
     const uint32_t sms = static_cast<uint32_t>(ctx->sm_count);
-    const uint32_t columns = geglu ? n / 2 : n;            // GEGLU: a tile holds t/2 value + t/2 gate columns
+    const uint32_t columns = ep.n_out;                     // GEGLU: a tile holds t/2 value + t/2 gate columns
     // `siblings`: problems of (about) this shape that share the launch (a small inline group)
     const uint64_t tiles_at_widest = static_cast<uint64_t>(siblings) * tiles_m * ((columns + (geglu ? 127 : 255)) / (geglu ? 128 : 256));
     const bool traffic_bound = grouped ? tiles_m >= 2 : tiles_at_widest >= 3ull * sms;
-    // CTA pairs halve the weight bytes per SM. Chosen for GEGLU launches of many tiles, and in launches of few for a K of
-    // at least 32 stages, or 20 from 4096 rows on (us, single CTAs against pairs, FP8 | FP16): GEGLU [2048, 10240],
-    // K = 1280: 26.6, 24.0 | 43.6, 39.6; [8192, 5120], K = 640: 37.0, 34.2 | 46.3, 41.3; [140, 1280], K = 5120: 11.4, 10.9 |
-    // 21.2, 19.1; [2048, 1280], K = 5120: 14.6, 13.8 | 23.9, 21.6; [8192, 640], K = 2560: 15.7, 14.7 | 25.6, 23.1. Not
-    // for shorter K (FP16 [1000, 1280], K = 1280, 20 stages: 11.7, 11.8, its q/k/v 11.6, 12.5), not for launches of many
-    // tiles without GEGLU (FP16 [65536, 640], K = 640: 79, 91), and not in plans, whose tiles would be split over two
-    // launches. set_pair_mode makes it never, always or by traffic.
-    bool pair_allowed = ctx->pair_mode != 0 && m > kTileM && (traffic_bound || ctx->pair_mode == 1);
-    if (ctx->pair_mode == kPairChosen) {
-        pair_allowed = allow_chosen_pairs && !grouped && ctx->forced_tile_n == 0 && m > kTileM && (geglu ? traffic_bound : !traffic_bound && k_blocks >= (m < 4096 ? 32u : 20u));
-    }
+    // set_pair_mode: never, always or by traffic
+    const bool pair_forced = ctx->pair_mode != kPairChosen && ctx->pair_mode != 0 && ep.m > kTileM && (traffic_bound || ctx->pair_mode == 1);
     if (ctx->forced_tile_n >= 16) {
         const uint32_t forced = std::min<uint32_t>(kMaxTileN, static_cast<uint32_t>(ctx->forced_tile_n));
         const uint32_t pair_step = 32;
-        if (pair_allowed) return TileChoice{std::max(pair_step, forced / pair_step * pair_step), true};
+        if (pair_forced) return TileChoice{std::max(pair_step, forced / pair_step * pair_step), true};
         return TileChoice{std::max(step, forced / step * step), false};
     }
     // Tuning override for the epilogue-heavy GEGLU tiles of a grouped launch (see geglu_tile_n).
-    if (geglu && grouped && ctx->geglu_tile_n >= 32 && !pair_allowed) {
+    if (geglu && grouped && ctx->geglu_tile_n >= 32 && !pair_forced) {
         return TileChoice{std::min<uint32_t>(kMaxTileN, static_cast<uint32_t>(ctx->geglu_tile_n) / 32u * 32u), false};
     }
-    TileChoice best{step, false};
-    double best_cost = 1e300;
-    for (int pair = pair_allowed ? 1 : 0; pair >= 0; --pair) {
+    const auto widest_best = [&](bool pair, bool by_traffic, uint64_t& best_waves) {
         const uint32_t tile_step = pair ? 32 : step;
+        const uint64_t workers = pair ? sms / 2 : sms;
+        uint32_t best = tile_step;
+        double best_cost = 1e300;
         for (uint32_t tile_n = kMaxTileN; tile_n >= tile_step; tile_n -= tile_step) {
             const uint32_t per_tile = geglu ? tile_n / 2 : tile_n;
             const uint32_t tiles_n = (columns + per_tile - 1) / per_tile;
-            double cost;
-            if (traffic_bound || (pair && ctx->pair_mode != kPairChosen)) {
-                cost = static_cast<double>(tiles_n) * (128.0 + (pair ? tile_n / 2.0 : tile_n));
-            } else {
-                const uint64_t workers = pair ? sms / 2 : sms;
-                const uint64_t tiles = static_cast<uint64_t>(siblings) * (pair ? (tiles_m + 1) / 2 : tiles_m) * tiles_n;
-                const uint64_t waves = (tiles + workers - 1) / workers;
-                cost = static_cast<double>(waves) * (tile_n + 32.0);
-            }
-            if (cost < best_cost) { best_cost = cost; best = TileChoice{tile_n, pair != 0}; }
+            const uint64_t tiles = static_cast<uint64_t>(siblings) * (pair ? (tiles_m + 1) / 2 : tiles_m) * tiles_n;
+            const uint64_t waves = (tiles + workers - 1) / workers;
+            const double cost = by_traffic ? static_cast<double>(tiles_n) * (128.0 + (pair ? tile_n / 2.0 : tile_n))
+                                           : static_cast<double>(waves) * (tile_n + 32.0);
+            if (cost < best_cost) { best_cost = cost; best = tile_n; best_waves = waves; }
             if (tile_n == tile_step) break;
         }
-        if (pair) break;      // a pair is allowed only where it wins: traffic-bound launches
+        return best;
+    };
+    uint64_t waves = 0;
+    if (pair_forced) return TileChoice{widest_best(true, true, waves), true};
+    const uint32_t single = widest_best(false, traffic_bound, waves);
+    if (ctx->pair_mode == kPairChosen && allow_chosen_pairs && !grouped &&
+        pairs_pay(ep.m, k_blocks, geglu, traffic_bound, waves, single)) {
+        // An odd number of row tiles leaves a pair half empty; not where that makes its tiles much wider than a single
+        // CTA's ([4736, 640], K = 8192: 148 tiles of 160 against 57 of 224: FP8 21.6, 24.6 us; FP16 52.8, 53.8).
+        uint64_t pair_waves = 0;
+        const uint32_t pair = widest_best(true, traffic_bound, pair_waves);
+        if (traffic_bound || pair_waves * (pair + 32) <= waves * (single + 64)) return TileChoice{pair, true};
     }
-    return best;
+    return TileChoice{single, false};
 }
 
 CUtensorMapDataType tensor_map_type(uint32_t kind) {
@@ -672,7 +689,7 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
     // K = 2048: 9.6, 16.2; INT8 [300, 1280], K = 1280 and K = 5120: 11.3, 15.6).
     const uint32_t siblings = grouped ? 1u : static_cast<uint32_t>(count);
     const auto tile_for = [&](const GemmCall& call, bool allow_chosen_pairs) {
-        return choose_tile(ctx, call.ep.m, call.ep.n, call.k_blocks, call.ep.activation == ACT_GEGLU, grouped, siblings, allow_chosen_pairs);
+        return choose_tile(ctx, call.ep, call.k_blocks, grouped, siblings, allow_chosen_pairs);
     };
     bool allow_chosen_pairs = true;
     if (!grouped && gemms.size() > 1) {

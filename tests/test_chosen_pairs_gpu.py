@@ -43,6 +43,28 @@ def test_same_bits_as_single_ctas(pkg, gpu_session, dtype, m, n, k, geglu):
     context.close()
 
 
+@pytest.mark.parametrize("m,n,k,activation,pairs", [
+    (128, 1280, 5120, "none", ""), (129, 1280, 5120, "none", "int8 e4m3 f16"), (300, 1280, 4096, "silu", "int8 e4m3 f16"),
+    (300, 1280, 3968, "none", "f16"), (300, 1280, 1984, "none", ""), (3000, 1280, 5120, "none", "f16"), (4000, 1280, 5120, "gelu", "int8 e4m3 f16"),
+    (5000, 640, 2560, "none", ""), (7000, 640, 2560, "none", "int8 e4m3 f16"), (3000, 1280, 4032, "none", ""), (7000, 640, 2432, "none", "f16"), (4736, 640, 8192, "none", ""), (8192, 640, 1216, "none", ""),
+    (1000, 5120, 640, "geglu", ""), (8192, 5120, 640, "geglu", "int8 e4m3 f16"), (65536, 640, 2560, "none", "")])
+def test_which_calls_take_pairs(pkg, gpu_session, m, n, k, activation, pairs):
+    """Both sides of the rule's lines, for a context whose pair mode was never set."""
+    context = pkg.Context(0, workspace_bytes=256 << 20)
+    ops = pkg.Ops(context)
+    x, bias = torch.zeros(m, k, device="cuda").half(), torch.zeros(n, device="cuda").half()
+    kinds = {"none": None, "silu": pkg.ACT_SILU, "gelu": pkg.ACT_GELU, "geglu": pkg.ACT_GEGLU}
+    for dtype in ("int8", "e4m3", "f16"):
+        weight = pack(pkg, ops, dtype, torch.ones(n, k, device="cuda").half())
+
+        def call():
+            return ops.linear(x, weight, bias) if activation == "none" else ops.linear_activation(x, weight, bias, kinds[activation])
+        gemms = [kernel for kernel in helpers.launches(context, call) if "umma_gemm" in kernel.name]
+        assert len(gemms) == 1 and (gemms[0].cluster == 2) == (dtype in pairs.split())
+    context.check()
+    context.close()
+
+
 @pytest.mark.parametrize("dtype", ["int8", "e4m3", "f16"])
 @pytest.mark.parametrize("shapes", [[(154, 1280, 1280), (154, 1280, 4096)], [(2048, 1280, 1280), (154, 1280, 4096), (154, 1280, 4096)],
                                     [(300, 1280, 5120), (300, 1280, 64)], [(257, 648, 5120), (300, 1280, 5120)]])
