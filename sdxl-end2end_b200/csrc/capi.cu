@@ -553,12 +553,15 @@ void choose_quantiser_block(const sdxlq_context* ctx, Int8JobSet& set) {
     }
 }
 
-// Single projections of at most kSkinnyRows rows (one row tile of that kernel's MMA) take the kernel that splits K over
-// warps; figures at linear_skinny.cu. It loads operands 16 bytes at a time; a forced tile shape asks for the other kernel.
+// Single projections of at most kSkinnyRows rows (one row tile of that kernel's MMA) can take the kernel that splits K over
+// warps (linear_skinny.cu); a forced tile shape or pair mode asks for the tensor-memory GEMM.
 constexpr uint64_t kSkinnyRows = 16;
-// Every block reads the whole FP16 input when it quantises for itself: up to 256 KB of it, and INT8 rows of the length
-// that the stand-alone quantiser takes.
-constexpr uint64_t kSkinnyInput = 131072, kSkinnyInt8Row = 16384;
+// Every block reads the whole FP16 input when it quantises for itself. INT8 rows are read twice and rounded in every block:
+// up to K = 1280 (us, own quantisation against the quantiser's launch in front: [1280, 640] 3.3, 3.9; [1280, 1280] 5.4 to
+// 5.7, 4.7 to 5.3, but one launch less of host time; [1280, 2048] 6.7, 5.1; 16 rows of K = 8192 23.0, 11.3). FP8 saves two
+// launches: up to 131072 values (8 rows [1280, 5120] 11.0, 11.3; [640, 8192] 9.6, 11.9; [1280, 8192] 16.0, 14.1; behind the
+// tensor-memory GEMM 17.8, 20.1, 23.9).
+constexpr uint64_t kSkinnyInput = 131072, kSkinnyInt8Row = 1280;
 
 bool overlap(const void* a, uint64_t a_bytes, const void* b, uint64_t b_bytes) {
     const uintptr_t first = reinterpret_cast<uintptr_t>(a), second = reinterpret_cast<uintptr_t>(b);
@@ -580,11 +583,24 @@ bool skinny_call(const sdxlq_context* ctx, const sdxlq_linear_desc& d, size_t co
            (w.dtype == SDXLQ_FP16 || d.xq == nullptr || outputs_apart(d, d.xq, d.m * w.k));
 }
 
-bool skinny_quantises(const sdxlq_linear_desc& d) {
+// Whether the kernel beats the tensor-memory GEMM (and its quantiser) for the call's columns: always while its blocks of 32
+// columns are at most one per SM. Beyond that the results of a block add up, and every block reads its activations again.
+// us, 8 / 16 rows against the GEMM: FP16 [5120], K = 1280 7.0 / 8.3, 11.2; [10240] 10.0, 11.1 / 12.1, 11.7; [20480] 16.2, 13.0.
+// INT8 quantised before [5120], K = 640 5.5, 6.1 / 6.6, 6.1; [10240], K = 1280 9.7, 10.0 / 11.8, 9.8. FP8 quantising for
+// itself [5120], K = 1280 9.6, 10.3 / 10.9, 10.3; [10240] 14.4, 11.3; quantised before [5120] 12.4, 10.3.
+bool skinny_pays(const sdxlq_context* ctx, const sdxlq_linear_desc& d, bool from_half) {
+    const bool geglu = d.activation == SDXLQ_ACT_GEGLU, fp8 = is_fp8(d.weight.dtype);
+    const uint64_t n_out = geglu ? d.weight.n / 2 : d.weight.n, columns = geglu ? 16 : 32;
+    const uint64_t sms = static_cast<uint64_t>(ctx->sm_count), per_sm = ((n_out + columns - 1) / columns + sms - 1) / sms;
+    return per_sm <= 1 || (per_sm <= (from_half ? 2u : fp8 ? 1u : 3u) && d.m * n_out <= (d.weight.dtype == SDXLQ_FP16 ? 81920u : 61440u));
+}
+
+bool skinny_quantises(const sdxlq_context* ctx, const sdxlq_linear_desc& d) {
     const sdxlq_weight& w = d.weight;
-    return d.x_amax == nullptr && reinterpret_cast<uintptr_t>(d.x) % 16 == 0 && d.m * w.k <= kSkinnyInput &&
+    return w.dtype != SDXLQ_FP16 && d.xq == nullptr && d.x_amax == nullptr && reinterpret_cast<uintptr_t>(d.x) % 16 == 0 &&
            outputs_apart(d, d.x, d.m * w.k * 2) &&
-           (w.dtype != SDXLQ_INT8 || (w.convrot_group_size == 0 && w.k <= kSkinnyInt8Row));
+           (w.dtype == SDXLQ_INT8 ? w.convrot_group_size == 0 && w.k <= kSkinnyInt8Row : d.m * w.k <= kSkinnyInput) &&
+           skinny_pays(ctx, d, true);
 }
 
 int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bool grouped, Prepared& prep) {
@@ -602,8 +618,9 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
                               : w.dtype == SDXLQ_FP8_E5M2 ? KIND_E5M2 : KIND_F16;
         const void* a = d.x;
         const float* a_scales = nullptr;
-        const bool skinny = skinny_call(ctx, d, count, grouped);
-        bool from_half = false;
+        const bool few_rows = skinny_call(ctx, d, count, grouped);
+        const bool from_half = few_rows && skinny_quantises(ctx, d);
+        const bool skinny = from_half || (few_rows && skinny_pays(ctx, d, false));
         if (kind == KIND_I8 || kind == KIND_E4M3 || kind == KIND_E5M2) {
             if (d.xq != nullptr) {
                 a = d.xq;
@@ -623,8 +640,8 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
                     }
                     uint8_t* q = ctx->workspace + q_offset;
                     float* s = reinterpret_cast<float*>(ctx->workspace + s_offset);
-                    if (skinny && skinny_quantises(d)) {
-                        from_half = true;                       // no quantiser launch
+                    if (from_half) {
+                        // no quantiser launch
                     } else if (kind == KIND_I8) {
                         const int job_status = add_int8_job(ctx, prep, d.x, false, d.m, w.k, w.convrot_group_size,
                                                             reinterpret_cast<int8_t*>(q), s, grouped);

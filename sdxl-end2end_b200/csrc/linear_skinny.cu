@@ -303,7 +303,8 @@ namespace {
 
 template <int kKind, bool kFromHalf>
 cudaError_t launch_groups(const SkinnyParams& params, uint32_t sm_count, cudaStream_t stream, bool early_launch) {
-    // As few columns per block as keep the grid within two blocks per SM: every block reads all of X.
+    // As few columns per block as keep the grid within two blocks per SM, which fit with one or two groups (at most 58
+    // registers; with four, 102 registers leave room for one block, 64 in INT8 for two). Every block reads all of X.
     const uint32_t halves = params.ep.activation == ACT_GEGLU ? 2 : 1;          // value and gate columns
     const uint32_t column_groups = (params.ep.n_out + 7) / 8;
     uint32_t out_groups = 1;

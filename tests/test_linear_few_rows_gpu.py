@@ -4,6 +4,8 @@ sum no larger than the sum S of the products' magnitudes, then the FP16 rounding
 import pytest
 import torch
 
+import helpers
+
 pytestmark = pytest.mark.gpu
 
 
@@ -107,3 +109,24 @@ def test_projection_in_place(gpu, dtype, m, k, shift):
         ops.linear(x, weight, bias, residual=x if with_residual else None, out=out)
         assert torch.equal(out, want if with_residual else ops.linear(values, weight, bias))
     ctx.check()
+
+
+@pytest.mark.parametrize("dtype,m,n,k,activation,expected", [
+    ("f16", 16, 4736, 64, "none", "skinny"), ("f16", 16, 5120, 64, "none", "skinny"), ("f16", 17, 64, 64, "none", "gemm"),
+    ("f16", 8, 10240, 64, "none", "skinny"), ("f16", 9, 10240, 64, "none", "gemm"), ("f16", 16, 10240, 64, "geglu", "skinny"), ("f16", 1, 20480, 64, "none", "gemm"),
+    ("int8", 16, 4736, 1280, "none", "skinny"), ("int8", 12, 5120, 64, "none", "skinny"), ("int8", 13, 5120, 64, "none", "quantiser gemm"),
+    ("int8", 2, 9504, 64, "none", "quantiser skinny"), ("int8", 16, 64, 1296, "none", "quantiser skinny"), ("int8256", 6, 10240, 256, "none", "quantiser skinny"),
+    ("int8256", 7, 10240, 256, "none", "quantiser gemm"), ("e4m3", 16, 4736, 64, "none", "skinny"), ("e4m3", 12, 5120, 64, "none", "skinny"),
+    ("e5m2", 13, 5120, 64, "none", "quantiser quantiser gemm"), ("e4m3", 1, 9504, 64, "none", "quantiser quantiser gemm"), ("e4m3", 16, 64, 8208, "none", "quantiser quantiser skinny"),
+    ("e4m3", 16, 64, 8192, "none", "skinny"), ("e4m3", 8, 10240, 64, "geglu", "quantiser quantiser gemm")])
+def test_which_calls_take_the_few_row_kernel(gpu, dtype, m, n, k, activation, expected):
+    """Both sides of the rule's lines, on 148 SMs."""
+    pkg, ctx, ops = gpu
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the sizes are those of 148 SMs")
+    weight = make(pkg, ops, dtype, n, k, torch.ones(n, k, device="cuda").half())
+    x, bias = torch.zeros(m, k, device="cuda").half(), torch.zeros(n, device="cuda").half()
+    kernels = helpers.launches(ctx, lambda: ops.linear(x, weight, bias) if activation == "none" else ops.linear_activation(x, weight, bias, pkg.ACT_GEGLU))
+    families = {"skinny": "skinny", "umma_gemm": "gemm", "fp8_amax": "quantiser", "fp8_cast": "quantiser", "plain_rows": "quantiser", "rotated": "quantiser"}
+    found = [family for kernel in kernels for part, family in families.items() if part in kernel.name]
+    assert sorted(found) == sorted(expected.split())
