@@ -71,14 +71,25 @@ private:
 
 bool is_none(PyObject* object) { return object == nullptr || object == Py_None; }
 
-// The tensor behind `object`: false when it is not a CUDA tensor. `pointer` stays null for None.
-bool optional_pointer(PyObject* object, void*& pointer) {
+// The tensor behind `object` (an input): false when it is not a CUDA tensor. `pointer` stays null for None.
+bool optional_input(PyObject* object, const void*& pointer) {
     pointer = nullptr;
     if (is_none(object)) return true;
     if (!THPVariable_Check(object)) return false;
     const at::Tensor& tensor = THPVariable_Unpack(object);
     if (!tensor.is_cuda()) return false;
-    pointer = const_cast<void*>(tensor.const_data_ptr());
+    pointer = tensor.const_data_ptr();
+    return true;
+}
+
+// The same for a tensor that the call writes. A copy-on-write tensor gets its own memory here.
+bool optional_output(PyObject* object, void*& pointer) {
+    pointer = nullptr;
+    if (is_none(object)) return true;
+    if (!THPVariable_Check(object)) return false;
+    const at::Tensor& tensor = THPVariable_Unpack(object);
+    if (!tensor.is_cuda()) return false;
+    pointer = tensor.mutable_data_ptr();
     return true;
 }
 
@@ -98,14 +109,14 @@ bool read_weight(PyObject* object, sdxlq_weight& w) {
     uint64_t type, layout, mode, group;
     {
         const Attribute data(object, g_names.data);
-        void* pointer = nullptr;
-        if (is_none(data.get()) || !optional_pointer(data.get(), pointer)) return false;
+        const void* pointer = nullptr;
+        if (is_none(data.get()) || !optional_input(data.get(), pointer)) return false;
         w.data = pointer;
     }
     {
         const Attribute scales(object, g_names.scales);
-        void* pointer = nullptr;
-        if (!optional_pointer(scales.get(), pointer)) return false;
+        const void* pointer = nullptr;
+        if (!optional_input(scales.get(), pointer)) return false;
         w.scales = static_cast<const float*>(pointer);
         w.scale_count = pointer == nullptr ? 0 : static_cast<uint64_t>(THPVariable_Unpack(scales.get()).numel());
     }
@@ -132,7 +143,8 @@ bool describe(const LinearArguments& a, bool poison, sdxlq_linear_desc& d, at::T
     d = sdxlq_linear_desc{};
     if (!read_weight(a.weight, d.weight)) return false;
     const int64_t k = static_cast<int64_t>(d.weight.k), n = static_cast<int64_t>(d.weight.n);
-    void *pointer = nullptr;
+    const void* input = nullptr;
+    void* output = nullptr;
     PyObject* const leading = is_none(a.input) ? a.xq : a.input;
     if (!ordinary(leading)) return false;
     const at::Tensor& lead = THPVariable_Unpack(leading);
@@ -157,16 +169,16 @@ bool describe(const LinearArguments& a, bool poison, sdxlq_linear_desc& d, at::T
         d.residual = residual.const_data_ptr();
     }
     d.activation = static_cast<int32_t>(a.activation);
-    if (!optional_pointer(a.xq, pointer)) return false;
-    d.xq = pointer;
-    if (!optional_pointer(a.xq_scales, pointer)) return false;
-    d.xq_scales = static_cast<const float*>(pointer);
-    if (!optional_pointer(a.acc_out, pointer)) return false;
-    d.acc_out = static_cast<int32_t*>(pointer);
-    if (!optional_pointer(a.y_amax, pointer)) return false;
-    d.y_amax = pointer;
-    if (!optional_pointer(a.x_amax, pointer)) return false;
-    d.x_amax = pointer;
+    if (!optional_input(a.xq, input)) return false;
+    d.xq = input;
+    if (!optional_input(a.xq_scales, input)) return false;
+    d.xq_scales = static_cast<const float*>(input);
+    if (!optional_output(a.acc_out, output)) return false;
+    d.acc_out = static_cast<int32_t*>(output);
+    if (!optional_output(a.y_amax, output)) return false;
+    d.y_amax = output;
+    if (!optional_output(a.x_amax, output)) return false;          // put back to zero by the call
+    d.x_amax = output;
     if (is_none(a.out)) {
         c10::SmallVector<int64_t, 5> sizes(lead.sizes().begin(), lead.sizes().end());
         sizes.back() = n_out;
@@ -174,8 +186,8 @@ bool describe(const LinearArguments& a, bool poison, sdxlq_linear_desc& d, at::T
         if (poison) allocated.fill_(std::numeric_limits<double>::quiet_NaN());
         d.y = allocated.mutable_data_ptr();
     } else {
-        if (!optional_pointer(a.out, pointer)) return false;
-        d.y = pointer;
+        if (!optional_output(a.out, output)) return false;
+        d.y = output;
     }
     return true;
 }
@@ -289,7 +301,7 @@ PyObject* layer_norm(PyObject*, PyObject* const* args, Py_ssize_t count) {
         if (is_none(args[5])) {
             allocated = empty(x.sizes(), at::kHalf, x);
             d.y = allocated.mutable_data_ptr();
-        } else if (!optional_pointer(args[5], d.y)) {
+        } else if (!optional_output(args[5], d.y)) {
             Py_RETURN_NONE;
         }
         return answer(unlocked(g_layer_norm, context_of(args[0]), &d), tensor_or(args[5], allocated));

@@ -60,3 +60,29 @@ def test_front_leaves_errors_to_the_python_path(gpu):
         ops.linear(torch.zeros(8, 16, device="cuda", dtype=torch.float16), w)
     with pytest.raises(pkg.CudaError, match="requires a bias"):         # found by the library behind the front
         ops.linear_activation(torch.zeros(8, 32, device="cuda", dtype=torch.float16), w, None, pkg.ACT_SILU)
+
+
+def test_outputs_that_share_copy_on_write_storage(gpu):
+    """A tensor the call writes gets its own memory; the tensor it was lazily cloned from keeps its values."""
+    pkg, ctx, ops = gpu
+    torch.manual_seed(4)
+    weight = ops.upload_or_quantize_int8_weight(torch.randn(64, 64, device="cuda"), None, pkg.INT8WeightLoadOptions(enable_convrot=False))
+    fp8 = ops.upload_fp8_weight(torch.randn(64, 64, device="cuda"), pkg.FP8WeightLoadOptions())
+    x, ones = torch.randn(20, 64, device="cuda").half(), torch.ones(64, device="cuda").half()
+    kept = {"y": torch.full((20, 64), 3.0, device="cuda", dtype=torch.float16), "acc": torch.full((20, 64), 3, device="cuda", dtype=torch.int32),
+            "amax": torch.zeros(1, device="cuda", dtype=torch.int32)}
+    before = {name: t.clone() for name, t in kept.items()}
+    clones = [{name: torch._lazy_clone(t) for name, t in kept.items()} for _ in range(4)]
+    assert ops.linear(x, weight, out=clones[0]["y"], acc_out=clones[0]["acc"], y_amax=clones[0]["amax"]) is clones[0]["y"]
+    ops.linear_grouped([pkg.LinearCall(x, weight, y=clones[1]["y"])])
+    ops.layer_norm(x, ones, ones, out=clones[2]["y"])
+    assert clones[0]["amax"].item() != 0 and not torch.equal(clones[0]["acc"], before["acc"])
+    word = clones[0]["amax"]
+    shared = torch._lazy_clone(word)
+    left = shared.item()
+    ops.linear(clones[0]["y"], fp8, x_amax=word)                   # reads the word and puts it back to zero
+    ctx.check()
+    assert word.item() == 0 and shared.item() == left
+    assert not any(torch.equal(clones[i]["y"], before["y"]) for i in range(3))
+    for name, t in kept.items():
+        assert torch.equal(t, before[name])
