@@ -101,7 +101,13 @@ bool half_vector(PyObject* object, int64_t width) {
     return t.scalar_type() == at::kHalf && t.dim() == 1 && t.size(0) == width && t.is_contiguous();
 }
 
+// Goes through the dispatcher where somebody may listen: a dispatch mode or a transform is active on this thread, or new
+// memory is filled for determinism. Otherwise straight to the allocator.
 at::Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const at::Tensor& like) {
+    const bool filled = at::globalContext().deterministicAlgorithms() && at::globalContext().deterministicFillUninitializedMemory();
+    if (filled || !(c10::impl::tls_local_dispatch_key_set().included_ == c10::default_included_set)) {
+        return at::empty(sizes, at::TensorOptions().dtype(type).device(like.device()));
+    }
     return at::Tensor(at::detail::empty_cuda(sizes, type, like.device(), std::nullopt));
 }
 

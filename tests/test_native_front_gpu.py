@@ -3,6 +3,8 @@ of argument, and the front hands over what it does not take, so that errors keep
 import pytest
 import torch
 
+import helpers
+
 pytestmark = pytest.mark.gpu
 
 
@@ -86,3 +88,36 @@ def test_outputs_that_share_copy_on_write_storage(gpu):
     assert not any(torch.equal(clones[i]["y"], before["y"]) for i in range(3))
     for name, t in kept.items():
         assert torch.equal(t, before[name])
+
+
+def test_outputs_are_allocated_through_the_dispatcher(gpu):
+    """A dispatch mode sees the allocations, and deterministic mode fills them, as on the Python path."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    pkg, ctx, ops = gpu
+    weight = ops.fp16_weight(torch.randn(64, 64, device="cuda").half())
+    x, ones = torch.randn(4, 64, device="cuda").half(), torch.ones(64, device="cuda").half()
+
+    class Record(TorchDispatchMode):
+        seen = 0
+
+        def __torch_dispatch__(self, function, types, args=(), kwargs=None):
+            Record.seen += "empty" in str(function)
+            return function(*args, **(kwargs or {}))
+
+    plain = pkg.Ops(ctx)
+    with Record():
+        plain.linear(x, weight)
+        plain.linear_grouped([pkg.LinearCall(x, weight), pkg.LinearCall(x, weight)])
+        plain.layer_norm(x, ones, ones)
+        plain.quantize_int8(x, 0)
+        plain.quantize_e4m3(x)
+    assert Record.seen == 1 + 2 + 1 + 2 + 2
+
+    assert not any("Fill" in kernel.name for kernel in helpers.launches(ctx, lambda: plain.linear(x, weight)))
+    torch.use_deterministic_algorithms(True)
+    try:
+        kernels = helpers.launches(ctx, lambda: plain.linear(x, weight))
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert any("Fill" in kernel.name for kernel in kernels)
+    ctx.check()
