@@ -27,6 +27,7 @@
 
 #include <cmath>
 #include <limits>
+#include <utility>
 
 namespace {
 
@@ -67,6 +68,20 @@ public:
 
 private:
     PyObject* value_;
+};
+
+// A reference that is released at the end of the scope, by an exception too, unless it was handed on.
+class Owned {
+public:
+    explicit Owned(PyObject* object) : object_(object) {}
+    ~Owned() { Py_XDECREF(object_); }
+    Owned(const Owned&) = delete;
+    Owned& operator=(const Owned&) = delete;
+    PyObject* get() const { return object_; }
+    PyObject* release() { return std::exchange(object_, nullptr); }
+
+private:
+    PyObject* object_;
 };
 
 bool is_none(PyObject* object) { return object == nullptr || object == Py_None; }
@@ -239,8 +254,8 @@ PyObject* linear_grouped(PyObject*, PyObject* const* args, Py_ssize_t count) {
     if (calls == 0 || calls > kMost) Py_RETURN_NONE;
     sdxlq_linear_desc descs[kMost];
     at::Tensor allocated[kMost];
-    PyObject* outputs = PyList_New(calls);
-    if (outputs == nullptr) return nullptr;
+    Owned outputs(PyList_New(calls));
+    if (outputs.get() == nullptr) return nullptr;
     for (Py_ssize_t i = 0; i < calls; ++i) {
         PyObject* const call = PyList_GET_ITEM(args[1], i);
         const Attribute x(call, g_names.x), weight(call, g_names.weight), bias(call, g_names.bias), y(call, g_names.y),
@@ -250,26 +265,21 @@ PyObject* linear_grouped(PyObject*, PyObject* const* args, Py_ssize_t count) {
                           residual.get(), y_amax.get(), x_amax.get(), 0};
         if (weight.get() == nullptr || !Attribute(call, g_names.activation).integer(a.activation) ||
             !describe(a, args[2] == Py_True, descs[i], allocated[i])) {
-            Py_DECREF(outputs);
             Py_RETURN_NONE;
         }
-        PyList_SET_ITEM(outputs, i, Py_NewRef(is_none(y.get()) ? Py_None : y.get()));
+        PyList_SET_ITEM(outputs.get(), i, Py_NewRef(is_none(y.get()) ? Py_None : y.get()));
     }
     const int status = unlocked(g_linear_grouped, context_of(args[0]), descs, static_cast<size_t>(calls));
-    if (status != SDXLQ_OK) return answer(status, outputs);
+    if (status != SDXLQ_OK) return PyLong_FromLong(status);
     for (Py_ssize_t i = 0; i < calls; ++i) {
         if (!allocated[i].defined()) continue;
-        PyObject* const y = THPVariable_Wrap(std::move(allocated[i]));
-        if (y == nullptr || PyObject_SetAttr(PyList_GET_ITEM(args[1], i), g_names.y, y) != 0) {
-            Py_XDECREF(y);
-            Py_DECREF(outputs);
-            return nullptr;
-        }
-        PyObject* const placeholder = PyList_GET_ITEM(outputs, i);
-        PyList_SET_ITEM(outputs, i, y);
+        Owned y(THPVariable_Wrap(std::move(allocated[i])));
+        if (y.get() == nullptr || PyObject_SetAttr(PyList_GET_ITEM(args[1], i), g_names.y, y.get()) != 0) return nullptr;
+        PyObject* const placeholder = PyList_GET_ITEM(outputs.get(), i);
+        PyList_SET_ITEM(outputs.get(), i, y.release());
         Py_DECREF(placeholder);
     }
-    return outputs;
+    return outputs.release();
 }
 
 PyObject* pair_of(at::Tensor& first, at::Tensor& second) {
