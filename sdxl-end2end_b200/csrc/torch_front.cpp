@@ -84,13 +84,14 @@ private:
     PyObject* object_;
 };
 
-bool is_none(PyObject* object) { return object == nullptr || object == Py_None; }
+bool is_none(PyObject* object) { return object == Py_None; }
 
-// The tensor behind `object` (an input): false when it is not a CUDA tensor. `pointer` stays null for None.
+// The tensor behind `object` (an input): false when it is not a CUDA tensor, or an attribute that does not exist. `pointer`
+// stays null for None.
 bool optional_input(PyObject* object, const void*& pointer) {
     pointer = nullptr;
     if (is_none(object)) return true;
-    if (!THPVariable_Check(object)) return false;
+    if (object == nullptr || !THPVariable_Check(object)) return false;
     const at::Tensor& tensor = THPVariable_Unpack(object);
     if (!tensor.is_cuda()) return false;
     pointer = tensor.const_data_ptr();
@@ -101,7 +102,7 @@ bool optional_input(PyObject* object, const void*& pointer) {
 bool optional_output(PyObject* object, void*& pointer) {
     pointer = nullptr;
     if (is_none(object)) return true;
-    if (!THPVariable_Check(object)) return false;
+    if (object == nullptr || !THPVariable_Check(object)) return false;
     const at::Tensor& tensor = THPVariable_Unpack(object);
     if (!tensor.is_cuda()) return false;
     pointer = tensor.mutable_data_ptr();

@@ -121,3 +121,16 @@ def test_outputs_are_allocated_through_the_dispatcher(gpu):
         torch.use_deterministic_algorithms(False)
     assert any("Fill" in kernel.name for kernel in kernels)
     ctx.check()
+
+
+@pytest.mark.parametrize("missing", ["bias", "residual", "acc_out", "y", "x_amax"])
+def test_front_leaves_incomplete_objects_to_the_python_path(gpu, missing):
+    """An attribute that does not exist is not None."""
+    from types import SimpleNamespace
+    pkg, ctx, ops = gpu
+    weight = ops.fp16_weight(torch.zeros(64, 32, device="cuda"))
+    call = vars(pkg.LinearCall(torch.zeros(4, 32, device="cuda").half(), weight))
+    with pytest.raises(AttributeError):
+        ops.linear_grouped([SimpleNamespace(**{name: value for name, value in call.items() if name != missing})])
+    with pytest.raises(AttributeError):
+        ops.linear(call["x"], SimpleNamespace(**{name: value for name, value in vars(weight).items() if name != "scales"}))
