@@ -253,6 +253,11 @@ PyObject* linear_grouped(PyObject*, PyObject* const* args, Py_ssize_t count) {
     if (count != 3 || !PyList_Check(args[1])) Py_RETURN_NONE;
     const Py_ssize_t calls = PyList_GET_SIZE(args[1]);
     if (calls == 0 || calls > kMost) Py_RETURN_NONE;
+    for (Py_ssize_t i = 1; i < calls; ++i) {
+        for (Py_ssize_t j = 0; j < i; ++j) {
+            if (PyList_GET_ITEM(args[1], i) == PyList_GET_ITEM(args[1], j)) Py_RETURN_NONE;      // one output for both
+        }
+    }
     sdxlq_linear_desc descs[kMost];
     at::Tensor allocated[kMost];
     Owned outputs(PyList_New(calls));

@@ -34,3 +34,10 @@ def test_an_exception_releases_the_list_of_outputs(pkg, front, fake):
         with pytest.raises(RuntimeError):
             front.linear_grouped(0, calls, False)
     assert lists() - before < 25
+
+
+def test_one_call_twice_is_left_to_the_python_path(pkg, front, fake):
+    """The two have one output between them."""
+    weight, x = fake
+    call = pkg.LinearCall(x, weight)
+    assert front.linear_grouped(0, [call, pkg.LinearCall(x, weight), call], False) is None
