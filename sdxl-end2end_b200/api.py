@@ -3,7 +3,10 @@ from __future__ import annotations
 
 import ctypes
 import enum
+import importlib.machinery
+import importlib.util
 import os
+import warnings
 from dataclasses import dataclass, field
 from typing import Optional, Sequence
 
@@ -201,16 +204,32 @@ _FRONT_FUNCTIONS = ("sdxlq_linear", "sdxlq_linear_grouped", "sdxlq_layer_norm", 
                     "sdxlq_quantize_act_fp8", "sdxlq_pack_weight_int8", "sdxlq_pack_weight_fp8")
 
 
+class _PythonPath:
+    """Stands in for a native front that is not there: answers None, so that the Python code issues every call."""
+
+    @staticmethod
+    def linear(*arguments):
+        return None
+
+    linear_grouped = layer_norm = quantize_int8 = quantize_fp8 = pack_fp8 = linear
+
+
 def load_front():
     """The native front (csrc/torch_front.cpp), bound to the loaded library. It issues ordinary calls without
-    ctypes; calls it does not take (it answers None) are checked and issued by the Python code below."""
+    ctypes; calls it does not take (it answers None) are checked and issued by the Python code below. Where it was
+    not built for this torch and Python, every call goes that way, with a warning."""
     global _front
     if _front is None:
         lib = load_library()
-        if not os.path.exists(_build.FRONT):
-            raise CudaError(f"{_build.FRONT} is missing: build it first (build() of this package, or "
-                            "__graft_entry__.build())", STATUS_CUDA)
-        from . import _front as module
+        try:
+            path = _build.front_path()
+            loader = importlib.machinery.ExtensionFileLoader(f"{__package__}._front", path)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader(loader.name, loader))
+            loader.exec_module(module)
+        except ImportError as error:
+            warnings.warn(f"no native front, calls go through ctypes (build() of this package makes it): {error}", RuntimeWarning)
+            _front = _PythonPath()
+            return _front
         module.bind(*(ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in _FRONT_FUNCTIONS))
         _front = module
     return _front
@@ -399,7 +418,7 @@ class Ops:
     def __init__(self, context: Context, poison_outputs: bool = False):
         self.ctx = context
         self._lib = context._lib
-        self._front = getattr(context, "_front", None)
+        self._front = getattr(context, "_front", None) or _PythonPath()
         # Tests set this: outputs this class allocates start as NaN, so that an element a kernel
         # failed to write cannot pass for a result left in recycled memory.
         self.poison_outputs = poison_outputs
