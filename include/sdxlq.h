@@ -312,11 +312,12 @@ size_t sdxlq_workspace_bytes(const sdxlq_linear_desc* descs, size_t count);
  * 0 restores the built-in choice). For tuning sweeps. */
 int sdxlq_context_set_tile_n(sdxlq_context* ctx, int tile_n);
 
-/* Selects the GEMM kernel flavour. Without this call single projections and small groups take CTA pairs
+/* Selects the GEMM kernel flavour. 2, the default: single projections and small groups take CTA pairs
  * (cta_group::2, 256-row tiles, each CTA loading half of the weight rows) where they measured faster. 0 runs
  * every tile on one CTA (128 rows); 1 uses pairs for every projection with more than 128 rows; -1 only for
  * projections of launches that fill the GPU several times over. Results are bit-identical between the
- * flavours. For tuning sweeps and tests. */
+ * flavours of that kernel; 1 and -1 also keep it for projections of at most 16 rows, which the other modes give to
+ * a kernel of their own (FP8 and FP16 sums in another order). For tuning sweeps and tests. */
 int sdxlq_context_set_pair_mode(sdxlq_context* ctx, int mode);
 
 /* Per-kernel device timing. While enabled, every kernel launch of the library is bracketed by a

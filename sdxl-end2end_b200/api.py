@@ -385,8 +385,8 @@ class Context:
         self.raise_for(self._lib.sdxlq_context_set_tile_n(self._handle, tile_n))
 
     def set_pair_mode(self, mode: int) -> None:
-        """CTA pairs: 0 never, 1 for every projection with more than 128 rows, -1 for launches that fill the GPU several
-        times over. Without this call: where they measured faster."""
+        """CTA pairs: 2 (the default) where they measured faster, 0 never, 1 for every projection with more than 128 rows,
+        -1 for launches that fill the GPU several times over."""
         self.raise_for(self._lib.sdxlq_context_set_pair_mode(self._handle, mode))
 
     def int8_execution_stats(self) -> dict:

@@ -1104,7 +1104,7 @@ int sdxlq_context_set_tile_n(sdxlq_context* ctx, int tile_n) {
 }
 
 int sdxlq_context_set_pair_mode(sdxlq_context* ctx, int mode) {
-    if (ctx == nullptr || mode < -1 || mode > 1) return SDXLQ_ERR_INVALID_ARGUMENT;
+    if (ctx == nullptr || mode < -1 || mode > kPairChosen) return SDXLQ_ERR_INVALID_ARGUMENT;
     ctx->pair_mode = mode;
     return SDXLQ_OK;
 }

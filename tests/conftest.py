@@ -43,6 +43,6 @@ def gpu_session(pkg):
 def gpu(gpu_session):
     """The session's context with the tuning switches a test may have left behind put back."""
     pkg, context, ops = gpu_session
-    context.set_pair_mode(0)
+    context.set_pair_mode(2)
     context.set_tile_n(0)
     return gpu_session

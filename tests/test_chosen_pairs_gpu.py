@@ -93,3 +93,23 @@ def test_a_small_group_is_one_launch(pkg, gpu_session, dtype, shapes):
         assert torch.equal(got, ops.linear(x, weight, **given))
     context.check()
     context.close()
+
+
+def test_the_default_choice_can_be_set_again(pkg, gpu):
+    _, context, ops = gpu
+    x = torch.zeros(300, 5120, device="cuda").half()
+    weights = [ops.fp16_weight(torch.zeros(1280, k, device="cuda")) for k in (5120, 64)]
+    inputs = [x, x[:, :64].contiguous()]
+
+    def pairs():
+        kernels = helpers.launches(context, lambda: [ops.linear(a, w) for a, w in zip(inputs, weights)])
+        return sorted(kernel.cluster for kernel in kernels if "umma_gemm" in kernel.name)
+
+    assert pairs() == [1, 2]
+    for mode, want in ((0, [1, 1]), (1, [2, 2]), (-1, [1, 1]), (2, [1, 2])):
+        context.set_pair_mode(mode)
+        assert pairs() == want
+    for mode in (-2, 3):
+        with pytest.raises(pkg.CudaError):
+            context.set_pair_mode(mode)
+    assert pairs() == [1, 2]
