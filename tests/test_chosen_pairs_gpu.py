@@ -1,6 +1,6 @@
 """Shapes for which single calls take CTA pairs by themselves (GEGLU of many tiles, a long K with few), at and beside
-the rule's edges: INT8 results equal those of single CTAs bit for bit, FP8 and FP16 too (the MMAs of a pair add the same
-products in the same order)."""
+the rule's edges: the results equal those of single CTAs bit for bit in every type (the MMAs of a pair add the same
+products in the same order), with every output and epilogue a call can ask for."""
 import pytest
 import torch
 
@@ -10,14 +10,16 @@ pytestmark = pytest.mark.gpu
 
 
 def pack(pkg, ops, dtype, source):
-    if dtype == "int8":
-        return ops.upload_or_quantize_int8_weight(source, None, pkg.INT8WeightLoadOptions(enable_convrot=False))
-    if dtype == "e4m3":
-        return ops.upload_fp8_weight(source, pkg.FP8WeightLoadOptions(scale_mode=pkg.FP8ScaleMode.PerOutputChannel))
-    return ops.fp16_weight(source)
+    if dtype.startswith("int8"):
+        group = int(dtype[4:] or 0)
+        return ops.upload_or_quantize_int8_weight(source, None, pkg.INT8WeightLoadOptions(enable_convrot=group != 0, convrot_group_size=group))
+    if dtype == "f16":
+        return ops.fp16_weight(source)
+    fmt = {"e4m3": pkg.ScalarType.Float8E4M3, "e5m2": pkg.ScalarType.Float8E5M2}[dtype]
+    return ops.upload_fp8_weight(source, pkg.FP8WeightLoadOptions(format=fmt, scale_mode=pkg.FP8ScaleMode.PerOutputChannel))
 
 
-@pytest.mark.parametrize("dtype", ["int8", "e4m3", "f16"])
+@pytest.mark.parametrize("dtype", ["int8", "int816", "e4m3", "e5m2", "f16"])
 @pytest.mark.parametrize("m,n,k,geglu", [(129, 64, 4096, False), (154, 1280, 5120, False), (257, 648, 4112, False), (2048, 1280, 3968, False), (4097, 640, 2560, False),
                                          (1976, 1280, 5120, False), (128, 1280, 5120, False), (3000, 5120, 640, True), (8192, 5120, 128, True),
                                          (1976, 10240, 1280, True)])
@@ -31,12 +33,17 @@ def test_same_bits_as_single_ctas(pkg, gpu_session, dtype, m, n, k, geglu):
     weight = pack(pkg, ops, dtype, (torch.randn(n, k, device="cuda") / k ** 0.5).half())
     x, bias = torch.randn(m, k, device="cuda").half(), torch.randn(n, device="cuda").half()
     for o in (ops, reference):
+        amax = torch.zeros(1, dtype=torch.int32, device="cuda")
         if geglu:
-            o.result = [o.linear_activation(x, weight, bias, pkg.ACT_GEGLU)]
+            o.result = [o.linear_activation(x, weight, bias, pkg.ACT_GEGLU, y_amax=amax), amax]
         else:
             residual = torch.randn(m, n, device="cuda", generator=torch.Generator("cuda").manual_seed(1)).half()
-            o.result = [o.linear(x, weight, bias), o.linear(x, weight, bias, residual=residual)]
+            o.result = [o.linear(x, weight, bias), o.linear(x, weight, bias, residual=residual, y_amax=amax), amax]
+            o.result += [o.linear_activation(x, weight, bias, activation) for activation in (pkg.ACT_SILU, pkg.ACT_GELU, pkg.ACT_QUICK_GELU)]
             o.result += o.linear_grouped([pkg.LinearCall(x, weight), pkg.LinearCall(x, weight, bias)])
+            if dtype.startswith("int8"):
+                accumulators = torch.zeros(m, n, dtype=torch.int32, device="cuda")
+                o.result += [o.linear(x, weight, acc_out=accumulators), accumulators]
     context.check()
     for got, want in zip(ops.result, reference.result):
         assert torch.equal(got, want)
