@@ -590,9 +590,9 @@ bool skinny_call(const sdxlq_context* ctx, const sdxlq_linear_desc& d, size_t co
 // itself [5120], K = 1280 9.6, 10.3 / 10.9, 10.3; [10240] 14.4, 11.3; quantised before [5120] 12.4, 10.3.
 bool skinny_pays(const sdxlq_context* ctx, const sdxlq_linear_desc& d, bool from_half) {
     const bool geglu = d.activation == SDXLQ_ACT_GEGLU, fp8 = is_fp8(d.weight.dtype);
-    const uint64_t n_out = geglu ? d.weight.n / 2 : d.weight.n, columns = geglu ? 16 : 32;
-    const uint64_t sms = static_cast<uint64_t>(ctx->sm_count), per_sm = ((n_out + columns - 1) / columns + sms - 1) / sms;
-    return per_sm <= 1 || (per_sm <= (from_half ? 2u : fp8 ? 1u : 3u) && d.m * n_out <= (d.weight.dtype == SDXLQ_FP16 ? 81920u : 61440u));
+    const uint32_t n_out = static_cast<uint32_t>(geglu ? d.weight.n / 2 : d.weight.n), columns = geglu ? 16 : 32;
+    const uint32_t blocks = (n_out + columns - 1) / columns, sms = static_cast<uint32_t>(ctx->sm_count);
+    return blocks <= sms || (blocks <= sms * (from_half ? 2u : fp8 ? 1u : 3u) && d.m * n_out <= (d.weight.dtype == SDXLQ_FP16 ? 81920u : 61440u));
 }
 
 bool skinny_quantises(const sdxlq_context* ctx, const sdxlq_linear_desc& d) {
@@ -678,7 +678,7 @@ int prepare(sdxlq_context* ctx, const sdxlq_linear_desc* descs, size_t count, bo
         ep.kind = kind;
         ep.activation = static_cast<uint32_t>(d.activation);
         ep.w_scale_per_channel = (kind != KIND_F16 && w.scale_count != 1) ? 1 : 0;
-        ep.vector_store_ok = row_access_ok(ep, 16);
+        ep.row_access = widest_row_access(ep);
         ep.vector_meta_ok = (reinterpret_cast<uintptr_t>(w.scales) % 16 == 0) &&
                             (reinterpret_cast<uintptr_t>(d.bias) % 16 == 0) &&
                             (!geglu || ep.n_out % 8 == 0);

@@ -41,14 +41,15 @@ struct EpilogueParams {
     uint32_t kind;               // GemmKind
     uint32_t activation;         // Activation
     uint32_t w_scale_per_channel;
-    uint32_t vector_store_ok;    // row_access_ok(.., 16)
+    uint32_t row_access;         // widest_row_access(..)
     uint32_t vector_meta_ok;     // w_scales / bias (and their GEGLU gate halves) are 16-byte aligned
 };
 
-// Whether the rows of y, and of the residual that is loaded the same way, take accesses of `bytes` bytes. The residual
-// has its own alignment: it need not alias y.
-__host__ __device__ inline bool row_access_ok(const EpilogueParams& ep, uint32_t bytes) {
-    return reinterpret_cast<uintptr_t>(ep.y) % bytes == 0 && reinterpret_cast<uintptr_t>(ep.residual) % bytes == 0 && ep.n_out % (bytes / 2) == 0;
+// Bytes (32, 16 or 2) of the widest access that the rows of y take, and those of the residual, which is loaded as wide as
+// y is stored and has its own alignment: it need not alias y.
+inline uint32_t widest_row_access(const EpilogueParams& ep) {
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(ep.y) | reinterpret_cast<uintptr_t>(ep.residual) | (uintptr_t(ep.n_out) * 2);
+    return bits % 32 == 0 ? 32 : bits % 16 == 0 ? 16 : 2;
 }
 
 // One GEMM problem of a grouped launch. Tensor maps first (64-byte alignment required).
@@ -110,10 +111,9 @@ __host__ __device__ inline TileRef make_tile_ref(const GemmProblem& problem, uin
     r.tile_n = static_cast<uint16_t>(problem.tile_n);
     r.kind = static_cast<uint8_t>(ep.kind);
     r.activation = static_cast<uint8_t>(ep.activation);
-    const bool store_32 = row_access_ok(ep, 32);
     r.flags = static_cast<uint16_t>((ep.bias != nullptr ? TILE_HAS_BIAS : 0) |
                                     (ep.kind != KIND_F16 && ep.w_scale_per_channel != 0 ? TILE_SCALE_PER_CHANNEL : 0) |
-                                    (ep.vector_store_ok != 0 ? TILE_STORE_16 : 0) | (store_32 ? TILE_STORE_32 : 0) |
+                                    (ep.row_access >= 16 ? TILE_STORE_16 : 0) | (ep.row_access >= 32 ? TILE_STORE_32 : 0) |
                                     (ep.acc_out != nullptr ? TILE_RAW_ACCUMULATORS : 0) |
                                     (ep.residual != nullptr ? TILE_HAS_RESIDUAL : 0) | (ep.y_amax != nullptr ? TILE_OUTPUT_AMAX : 0));
     r.m = ep.m;

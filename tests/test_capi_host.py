@@ -96,7 +96,7 @@ def test_row_accesses_follow_the_residual_too(pkg, tmp_path):
         "  p.ep.y = reinterpret_cast<__half*>(4096 + std::atoi(v[1]));\n"
         "  if (std::atoi(v[2]) >= 0) p.ep.residual = reinterpret_cast<__half*>(8192 + std::atoi(v[2]));\n"
         "  p.ep.n = p.ep.n_out = std::atoi(v[3]);\n"
-        "  p.ep.vector_store_ok = sdxlq::row_access_ok(p.ep, 16);\n"
+        "  p.ep.row_access = sdxlq::widest_row_access(p.ep);\n"
         "  const unsigned flags = sdxlq::make_tile_ref(p, 0, 0, 0).flags;\n"
         '  std::printf("%d", (flags & sdxlq::TILE_STORE_32) ? 32 : (flags & sdxlq::TILE_STORE_16) ? 16 : 2);\n'
         "}\n")
