@@ -81,7 +81,6 @@ struct sdxlq_context {
                                               // GEGLU epilogues but measured slower (operand traffic, per-tile costs).
     int pair_mode = kPairChosen;              // kPairChosen: where they measured faster (see pairs_pay); 0 never use
                                               // CTA pairs, 1 whenever possible, -1 for traffic-bound launches only
-    uint32_t diagnostic_skip = 0;             // SDXLQ_DIAGNOSTIC_SKIP: tuning aid, see GemmLaunchParams
     long long wait_limit_cycles = 4000000000LL;
     int forced_tile_n = 0;
     EncodeTiledFn encode = nullptr;
@@ -862,7 +861,6 @@ int run_gemm_flavour(sdxlq_context* ctx, const Prepared& prep, int flavour, cons
     params.b_offset = kTileM * kTileKBytes;
     params.error_word = ctx->control;
     params.wait_limit_cycles = ctx->wait_limit_cycles;
-    params.diagnostic_skip = ctx->diagnostic_skip;
     const uint32_t sms = static_cast<uint32_t>(ctx->sm_count);
     const uint32_t grid = pair ? 2 * std::min<uint32_t>(params.num_tiles, sms / 2) : std::min<uint32_t>(params.num_tiles, sms);
     // the kernel instance compiled for one operand class when every problem of the launch has it
@@ -1065,9 +1063,6 @@ int sdxlq_context_create(int device, void* stream, size_t workspace_bytes, sdxlq
     if (const char* text = std::getenv("SDXLQ_TILE_N")) ctx->forced_tile_n = std::atoi(text);
     if (const char* text = std::getenv("SDXLQ_PAIR")) ctx->pair_mode = std::atoi(text);
     if (const char* text = std::getenv("SDXLQ_GEGLU_TILE_N")) ctx->geglu_tile_n = std::atoi(text);
-#ifdef SDXLQ_DIAGNOSTICS
-    if (const char* text = std::getenv("SDXLQ_DIAGNOSTIC_SKIP")) ctx->diagnostic_skip = static_cast<uint32_t>(std::atoi(text));
-#endif
     if (const char* text = std::getenv("SDXLQ_EARLY_LAUNCH")) ctx->early_launch = std::atoi(text) != 0;
     if (const char* text = std::getenv("SDXLQ_QUANT_THREADS")) {
         const int threads = std::atoi(text);
@@ -1148,11 +1143,7 @@ int sdxlq_get_stats(const sdxlq_context* ctx, sdxlq_int8_stats* out) {
 int sdxlq_valid_convrot_group_size(size_t group_size) { return valid_group(group_size) ? 1 : 0; }
 
 const char* sdxlq_build_info(void) {
-#ifdef SDXLQ_DIAGNOSTICS
-    return "sdxlq sm_100a tcgen05/TMA cta_group::1 128xN + cta_group::2 256xN (diagnostic switches built in)";
-#else
     return "sdxlq sm_100a tcgen05/TMA cta_group::1 128xN + cta_group::2 256xN";
-#endif
 }
 
 size_t sdxlq_workspace_bytes(const sdxlq_linear_desc* descs, size_t count) {
@@ -1523,14 +1514,6 @@ int sdxlq_pack_weight_fp8(sdxlq_context* ctx, const void* src, int32_t src_dtype
     return SDXLQ_OK;
 }
 
-#ifdef SDXLQ_DIAGNOSTICS
-// Tuning build: the 64 control words (error word, then the GEMM kernel's cycle counters of its last launch).
-int sdxlq_debug_read_control(sdxlq_context* ctx, uint32_t* out) {
-    if (ctx == nullptr || out == nullptr) return SDXLQ_ERR_INVALID_ARGUMENT;
-    cudaStreamSynchronize(ctx->stream);
-    return cudaMemcpy(out, ctx->control, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost) == cudaSuccess ? SDXLQ_OK : SDXLQ_ERR_CUDA;
-}
-#endif
 
 int sdxlq_profile_enable(sdxlq_context* ctx, int enabled) {
     if (ctx == nullptr) return SDXLQ_ERR_INVALID_ARGUMENT;

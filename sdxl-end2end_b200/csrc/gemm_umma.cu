@@ -24,18 +24,6 @@
 
 namespace sdxlq {
 
-// Tuning build only: cycle counters of CTA 0's roles, written behind the error word (words 16..47 of the
-// control buffer) when the kernel ends. DIAG_ADD(counter, statement) times the statement.
-#ifdef SDXLQ_DIAGNOSTICS
-#define DIAG_DECL(name) long long name = 0
-#define DIAG_ADD(name, ...) do { const long long diag_t0 = clock64(); __VA_ARGS__; name += clock64() - diag_t0; } while (0)
-#define DIAG_WRITE(index, value) do { if (blockIdx.x == 0) params.error_word[16 + (index)] = static_cast<uint32_t>(value); } while (0)
-#else
-#define DIAG_DECL(name)
-#define DIAG_ADD(name, ...) do { __VA_ARGS__; } while (0)
-#define DIAG_WRITE(index, value)
-#endif
-
 namespace {
 
 constexpr uint32_t kMaxStages = 8;
@@ -303,7 +291,6 @@ struct EpilogueTile {
     uint32_t chunk_first;           // which of the warps of this TMEM lane quadrant
     uint32_t activation;            // Activation (read by the run-time activation variant)
     uint32_t flags;                 // bit 0 row in range, bit 1 has bias, bit 2 16-byte stores, bit 3 32-byte stores
-                                    // (bits 4-8: tuning switches of the diagnostics build)
 };
 
 // 16 accumulator columns of one row -> 16 FP16 outputs (no GEGLU): dequantise, bias, activation.
@@ -427,17 +414,8 @@ __device__ __forceinline__ void epilogue_tile(const EpilogueTile& t) {
     const float2 a_scale = make_float2(t.a_scale, t.a_scale);
     int32_t* const acc_out = Kind == KIND_I8 ? t.acc_out : nullptr;
     constexpr uint32_t kStride = kWarpsPerQuadrant * 16u;
-#ifdef SDXLQ_DIAGNOSTICS
-    // tuning build: parts of the epilogue can be switched off to time the others
-    const bool no_store = (t.flags & 16u) != 0, no_load = (t.flags & 32u) != 0, no_math = (t.flags & 64u) != 0;
-    if ((t.flags & 128u) != 0) return;                      // nothing at all
-    const uint32_t diag_limit = (t.flags & 256u) != 0 ? 32u : 0xFFFFFFFFu;     // one chunk per warp only
-#else
-    constexpr bool no_store = false, no_load = false, no_math = false;
-    constexpr uint32_t diag_limit = 0xFFFFFFFFu;
-#endif
     const uint32_t columns = Act == ACT_GEGLU ? t.tile_n / 2u : t.tile_n;        // output columns of the tile
-    const uint32_t limit = min(diag_limit, min(columns, t.n_out > t.n0 ? t.n_out - t.n0 : 0u));
+    const uint32_t limit = min(columns, t.n_out > t.n0 ? t.n_out - t.n0 : 0u);
     // max |y| over this lane's outputs of the tile, for the FP8 quantiser of the projection that reads y
     const bool want_amax = t.amax_out != nullptr;
     __half2 running_max = __float2half2_rn(0.0f);
@@ -447,13 +425,8 @@ __device__ __forceinline__ void epilogue_tile(const EpilogueTile& t) {
         uint32_t out_words[8];
         if (Act != ACT_GEGLU) {
             uint32_t acc[16];
-            if (no_load) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) acc[i] = c + t.row + static_cast<uint32_t>(i);
-            } else {
-                ptx::tmem_ld_32x32b_x16(t.tmem_row + c, acc);
-            }
-            if (!no_load) ptx::tmem_ld_wait(acc);
+            ptx::tmem_ld_32x32b_x16(t.tmem_row + c, acc);
+            ptx::tmem_ld_wait(acc);
             if (acc_out != nullptr && row_ok) {
                 int32_t* raw = acc_out + static_cast<size_t>(t.row) * t.n + col0;
 #pragma unroll
@@ -461,12 +434,7 @@ __device__ __forceinline__ void epilogue_tile(const EpilogueTile& t) {
                     if (col0 + i < t.n) raw[i] = static_cast<int32_t>(acc[i]);
                 }
             }
-            if (no_math) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) out_words[i] = acc[2 * i] ^ acc[2 * i + 1];
-            } else {
-                finish_chunk_16<Kind, Act>(t, c, acc, a_scale, has_bias, out_words);
-            }
+            finish_chunk_16<Kind, Act>(t, c, acc, a_scale, has_bias, out_words);
         } else {
             const uint32_t half = t.tile_n / 2u;
 #pragma unroll
@@ -488,9 +456,7 @@ __device__ __forceinline__ void epilogue_tile(const EpilogueTile& t) {
                 finish_geglu_8<Kind>(t, c + 8u * step, half, value, gate, a_scale, out_words + 4 * step);
             }
         }
-        if (row_ok && (!no_store || (out_words[0] == 0x7E57C0DEu && out_words[7] == 0x7E57C0DEu))) {
-            store_row_16(t.y, t.n_out, store_vector, store_wide, t.row, col0, out_words);
-        }
+        if (row_ok) store_row_16(t.y, t.n_out, store_vector, store_wide, t.row, col0, out_words);
         if (want_amax && row_ok) {
             // columns past the matrix edge hold zeros (scale 0, bias 0), so they cannot win the maximum
 #pragma unroll
@@ -579,7 +545,6 @@ struct MmaCursor {
     uint32_t stage_units, b_units;      // stage size and B offset in descriptor units (16 bytes)
     volatile uint32_t* abort_word;
     long long limit;
-    uint32_t mode;                      // diagnostics: bit 0 no MMAs, bit 1 one MMA per stage
 };
 
 // Issues the MMAs of one tile: k_blocks stages of four MMAs each, into the accumulator at tmem_d.
@@ -593,15 +558,7 @@ __device__ __forceinline__ bool issue_tile_mmas(MmaCursor& c, uint32_t tmem_d, u
         ptx::tc_fence_after();
         if (ptx::elect_one()) {
             const uint32_t a_lo = c.a_lo_base + stage * c.stage_units;
-            if (c.mode == 0) {
-                ptx::umma_stage<KindTag, kPair>(tmem_d, a_lo, a_lo + c.b_units, ptx::kUmmaDescHiSw128, idesc, accumulate);
-            } else if (c.mode == 2 && KindTag != 0) {   // the one-MMA diagnostic exists for INT8 only
-                ptx::umma_stage<KindTag, kPair>(tmem_d, a_lo, a_lo + c.b_units, ptx::kUmmaDescHiSw128, idesc, accumulate);
-            } else if (c.mode == 2) {
-                const uint64_t hi = static_cast<uint64_t>(ptx::kUmmaDescHiSw128) << 32;
-                if (kPair) ptx::umma_i8_pair(tmem_d, hi | a_lo, hi | (a_lo + c.b_units), idesc, accumulate);
-                else ptx::umma_i8(tmem_d, hi | a_lo, hi | (a_lo + c.b_units), idesc, accumulate);
-            }
+            ptx::umma_stage<KindTag, kPair>(tmem_d, a_lo, a_lo + c.b_units, ptx::kUmmaDescHiSw128, idesc, accumulate);
             const uint32_t empty_bar = c.empty_base + stage * 8u;
             if (kPair) {
                 ptx::umma_commit_pair(empty_bar);                                 // frees the leader's stage
@@ -645,18 +602,6 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
     const uint32_t num_tiles = params.num_tiles;
     volatile uint32_t* abort_word = &control->abort;
     const long long limit = params.wait_limit_cycles;
-#ifndef SDXLQ_DIAGNOSTICS
-    // regular build: the tuning switches do not exist and the hot loops carry no tests for them
-    // (1.5 % of the kernel time); build with -DSDXLQ_DIAGNOSTICS to get them
-    constexpr bool skip_epilogue = false, skip_loads = false, skip_mma = false, one_mma_per_stage = false,
-                   a_loads_only = false;
-#else
-    const bool skip_epilogue = (params.diagnostic_skip & 1u) != 0;
-    const bool skip_loads = (params.diagnostic_skip & (2u | 4u)) != 0;
-    const bool skip_mma = (params.diagnostic_skip & (2u | 8u)) != 0;
-    const bool one_mma_per_stage = (params.diagnostic_skip & 32u) != 0;
-    const bool a_loads_only = (params.diagnostic_skip & 64u) != 0;
-#endif
     const uint32_t cta_rank = kPair ? ptx::cluster_cta_rank() : 0u;
     const bool leader = cta_rank == 0;
     const uint32_t first_tile = kPair ? blockIdx.x >> 1 : blockIdx.x;
@@ -715,8 +660,6 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
             const GemmProblem* bound = nullptr;
             bool ok = true;
             TileRef next = load_tile(params, first_tile);
-            // diagnostic without loads: only the leader's arrivals count, its peer has nothing to do
-            if (kPair && skip_loads && !leader) ok = false;
             for (uint32_t t = first_tile; ok && t < num_tiles; t += tile_stride) {
                 const TileRef work = next;
                 next = load_tile(params, t + tile_stride);      // in flight while this tile's loads are issued
@@ -742,10 +685,8 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
                 // pair: this CTA's half of the B rows (GEGLU: value rows in the leader, gate rows in the peer)
                 const int32_t row_b_pair = geglu ? (leader ? row_b : row_gate)
                                                       : row_b + static_cast<int32_t>(cta_rank * half);
-                // diagnostic without loads and MMAs: no stage hand-shakes either, the epilogue runs alone
-                const uint32_t k_blocks = (skip_loads && skip_mma) ? 0u : work.k_blocks;
                 int32_t k0 = 0;
-                for (uint32_t kb = 0; kb < k_blocks; ++kb, k0 += k_step) {
+                for (uint32_t kb = 0; kb < work.k_blocks; ++kb, k0 += k_step) {
                     if (!ptx::warp_wait_bounded(empty_base + stage * 8u, phase ^ 1u, abort_word, limit)) {
                         raise_abort(control, params.error_word, DEV_TIMEOUT_PRODUCER);
                         ok = false;
@@ -755,15 +696,10 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
                     const uint32_t a_dst = stages_base + stage * stage_bytes;
                     const uint32_t b_dst = a_dst + b_offset;
                     if (ptx::elect_one()) {
-                        if (skip_loads) {
-                            if (leader) ptx::mbar_arrive(full_bar);
-                        } else if (kPair) {
+                        if (kPair) {
                             if (leader) ptx::mbar_expect_tx(full_bar, tx_bytes);
                             ptx::tma_load_2d_pair(a_dst, tmap_a, full_bar, k0, row_a);
                             ptx::tma_load_2d_pair(b_dst, tmap_b, full_bar, k0, row_b_pair);
-                        } else if (a_loads_only) {      // diagnostic: half of the copy instructions, a third of the bytes
-                            ptx::mbar_expect_tx(full_bar, kTileM * kTileKBytes);
-                            ptx::tma_load_2d(a_dst, tmap_a, full_bar, k0, row_a);
                         } else {
                             ptx::mbar_expect_tx(full_bar, tx_bytes);
                             ptx::tma_load_2d(a_dst, tmap_a, full_bar, k0, row_a);
@@ -775,7 +711,7 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
                     if (++stage == num_stages) { stage = 0; phase ^= 1u; }
                 }
             }
-            if (!ok && (!kPair || leader) && !skip_loads) {
+            if (!ok && (!kPair || leader)) {
                 // Let the copies this thread started land before the CTA retires: the last
                 // min(issued, num_stages) stages may still be in flight.
                 const uint32_t pending = min(issued, num_stages);
@@ -805,39 +741,27 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
             cursor.b_units = b_offset >> 4;
             cursor.abort_word = abort_word;
             cursor.limit = limit;
-            cursor.mode = (skip_mma ? 1u : 0u) | (one_mma_per_stage ? 2u : 0u);
             AccumulatorRing ring;
             bool ok = true;
-            DIAG_DECL(diag_acc_empty_wait); DIAG_DECL(diag_issue);
-#ifdef SDXLQ_DIAGNOSTICS
-            const long long diag_begin = clock64();
-#endif
             TileRef next = load_tile(params, first_tile);
             for (uint32_t t = first_tile; ok && t < num_tiles; t += tile_stride) {
                 const TileRef work = next;
                 next = load_tile(params, t + tile_stride);      // in flight while this tile's MMAs are issued
                 uint32_t quarters;
                 const uint32_t first_quarter = ring.place(work.tile_n, quarters);
-#ifdef SDXLQ_DIAGNOSTICS
-                const long long diag_t_wait = clock64();
-#endif
                 for (uint32_t q = first_quarter; ok && q < first_quarter + quarters; ++q) {
                     // the quarter's previous user (if any) has been drained by every epilogue warp
                     ok = ptx::warp_wait_bounded(ptx::smem_u32(&control->acc_empty[q]), ((ring.parity >> q) & 1u) ^ 1u,
                                                 abort_word, limit);
                     ring.parity ^= 1u << q;
                 }
-#ifdef SDXLQ_DIAGNOSTICS
-                const long long diag_t_issue = clock64();
-                diag_acc_empty_wait += diag_t_issue - diag_t_wait;
-#endif
                 if (!ok) {
                     raise_abort(control, params.error_word, DEV_TIMEOUT_MMA);
                     break;
                 }
                 ptx::tc_fence_after();
                 const uint32_t tmem_d = tmem_base + first_quarter * kQuarterColumns;
-                const uint32_t k_blocks = (skip_loads && skip_mma) ? 0u : work.k_blocks;
+                const uint32_t k_blocks = work.k_blocks;
                 if constexpr (kClass >= 0) {
                     ok = issue_tile_mmas<kClass, kPair>(cursor, tmem_d, work.idesc, k_blocks);
                 } else {
@@ -858,46 +782,30 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
                         ptx::umma_commit(full_bar);
                     }
                 }
-#ifdef SDXLQ_DIAGNOSTICS
-                diag_issue += clock64() - diag_t_issue;
-#endif
             }
-#ifdef SDXLQ_DIAGNOSTICS
-            DIAG_WRITE(4, diag_acc_empty_wait); DIAG_WRITE(5, diag_issue); DIAG_WRITE(6, clock64() - diag_begin);
-#endif
         }
     } else {
         // ------------------------------- stagers (warps 2 and 3) ---------------------------
         // Fill the epilogue's operand slot of each tile (tile record, row scales, column scales
         // and bias) while the tile's main loop runs, up to kSlots tiles ahead of the epilogue.
         uint32_t iteration = 0;
-        DIAG_DECL(diag_slot_wait); DIAG_DECL(diag_stage); DIAG_DECL(diag_total);
-#ifdef SDXLQ_DIAGNOSTICS
-        const long long diag_begin = clock64();
-#endif
         TileRef next = load_tile(params, first_tile);
         for (uint32_t t = first_tile; t < num_tiles; t += tile_stride, ++iteration) {
             const TileRef work = next;
             next = load_tile(params, t + tile_stride);
             const uint32_t slot = iteration % kSlots;
             uint32_t ok = 1;
-            DIAG_ADD(diag_slot_wait,
             if (lane == 0) {
                 ok = ptx::mbar_wait_bounded(ptx::smem_u32(&control->slot_free[slot]), ((iteration / kSlots) & 1u) ^ 1u,
                                             abort_word, limit) ? 1u : 0u;
                 if (ok == 0) raise_abort(control, params.error_word, DEV_TIMEOUT_EPILOGUE + 1);
             }
-            ok = __shfl_sync(0xffffffffu, ok, 0));
+            ok = __shfl_sync(0xffffffffu, ok, 0);
             if (ok == 0) break;
-            DIAG_ADD(diag_stage,
             stage_tile(work, work.tile_m * kRowsPerTile + cta_rank * kTileM, lane, warp - 2u, control, slot);
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&control->staged[slot])));
+            if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&control->staged[slot]));
         }
-#ifdef SDXLQ_DIAGNOSTICS
-        diag_total = clock64() - diag_begin;
-        if (warp == 2 && lane == 0) { DIAG_WRITE(0, diag_slot_wait); DIAG_WRITE(1, diag_stage); DIAG_WRITE(2, diag_total); DIAG_WRITE(3, iteration); }
-#endif
     }
     } else {
         // ------------------------------- epilogue ------------------------------------------
@@ -909,23 +817,12 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
         const uint32_t row_in_cta = quadrant * 32u + lane;
         AccumulatorRing ring;
         uint32_t iteration = 0;
-        DIAG_DECL(diag_staged_wait); DIAG_DECL(diag_acc_wait); DIAG_DECL(diag_work); DIAG_DECL(diag_setup); DIAG_DECL(diag_tail);
-#ifdef SDXLQ_DIAGNOSTICS
-        const long long diag_begin = clock64();
-#endif
         for (uint32_t t = first_tile; t < num_tiles; t += tile_stride, ++iteration) {
             const uint32_t buffer = iteration % kSlots;
-#ifdef SDXLQ_DIAGNOSTICS
-            const long long diag_t_staged = clock64();
-#endif
             if (!ptx::mbar_wait_bounded(ptx::smem_u32(&control->staged[buffer]), (iteration / kSlots) & 1u, abort_word, limit)) {
                 raise_abort(control, params.error_word, DEV_TIMEOUT_EPILOGUE);
                 break;
             }
-#ifdef SDXLQ_DIAGNOSTICS
-            const long long diag_t_setup = clock64();
-            diag_staged_wait += diag_t_setup - diag_t_staged;
-#endif
             const TileRef& work = control->header[buffer];
             const uint32_t tile_n = work.tile_n;
             const uint32_t activation = work.activation;
@@ -954,15 +851,7 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
             tile.activation = activation;
             tile.flags = (tile.row < work.m ? 1u : 0u) | ((flags & TILE_HAS_BIAS) != 0 ? 2u : 0u) |
                          ((flags & TILE_STORE_16) != 0 ? 4u : 0u) | ((flags & TILE_STORE_32) != 0 ? 8u : 0u);
-#ifdef SDXLQ_DIAGNOSTICS
-            tile.flags |= ((params.diagnostic_skip >> 7) & 31u) << 4;    // 128 no stores, 256 no accumulator loads, 512 no arithmetic,
-                                                                         // 1024 empty epilogue function, 2048 one chunk per warp
-#endif
             tile.a_scale = control->row_scale[buffer][row_in_cta];
-#ifdef SDXLQ_DIAGNOSTICS
-            const long long diag_t_acc = clock64();
-            diag_setup += diag_t_acc - diag_t_setup;
-#endif
             // the residual of this warp's first chunks travels while the accumulators are being completed
             const uint32_t residual_limit = min(tile_n, tile.n_out > tile.n0 ? tile.n_out - tile.n0 : 0u);
             uint32_t extra[kResidualDepth][8];
@@ -979,12 +868,7 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
             }
             ring.parity ^= 1u << first_quarter;
             ptx::tc_fence_after();
-#ifdef SDXLQ_DIAGNOSTICS
-            const long long diag_t_work = clock64();
-            diag_acc_wait += diag_t_work - diag_t_acc;
-#endif
-            if (skip_epilogue) { /* diagnostic: accumulators are dropped */ }
-            else if (tile.residual != nullptr) {
+            if (tile.residual != nullptr) {
                 if (kClass == 0 || (kClass < 0 && kind == KIND_I8)) epilogue_tile_residual<KIND_I8>(tile, residual_limit, extra);
                 else if (kClass == 2 || (kClass < 0 && kind == KIND_F16)) epilogue_tile_residual<KIND_F16>(tile, residual_limit, extra);
                 else epilogue_tile_residual<KIND_E4M3>(tile, residual_limit, extra);
@@ -995,10 +879,6 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
             else if (kind == KIND_I8) epilogue_dispatch<KIND_I8>(activation, tile);
             else if (kind == KIND_F16) epilogue_dispatch<KIND_F16>(activation, tile);
             else epilogue_dispatch<KIND_E4M3>(activation, tile);
-#ifdef SDXLQ_DIAGNOSTICS
-            const long long diag_t_tail = clock64();
-            diag_work += diag_t_tail - diag_t_work;
-#endif
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) {
@@ -1009,16 +889,7 @@ sdxlq_umma_gemm_kernel(const __grid_constant__ GemmLaunchParams params) {
                 }
                 ptx::mbar_arrive(ptx::smem_u32(&control->slot_free[buffer]));
             }
-#ifdef SDXLQ_DIAGNOSTICS
-            diag_tail += clock64() - diag_t_tail;
-#endif
         }
-#ifdef SDXLQ_DIAGNOSTICS
-        if (warp == kControlWarps && lane == 0) {
-            DIAG_WRITE(8, diag_staged_wait); DIAG_WRITE(9, diag_setup); DIAG_WRITE(10, diag_acc_wait); DIAG_WRITE(11, diag_work);
-            DIAG_WRITE(12, diag_tail); DIAG_WRITE(13, clock64() - diag_begin); DIAG_WRITE(14, iteration);
-        }
-#endif
     }
 
     ptx::tc_fence_before();

@@ -139,13 +139,9 @@ struct GemmLaunchParams {
     uint32_t b_offset;           // offset of the B tile inside a stage (= 128 rows * 128 B)
     uint32_t* error_word;        // device word set on a bounded-wait timeout
     long long wait_limit_cycles;
-    uint32_t diagnostic_skip;    // tuning aid, results are meaningless when set. bit 0: no epilogue arithmetic or
-                                 // stores; bit 1: no operand loads, no MMAs; bit 2: no operand loads; bit 3: no
-                                 // MMAs; bit 5: one MMA per stage instead
-                                 // of four; bit 6: only the A operand is loaded. Barriers are still signalled.
     uint32_t inline_count;       // problems in `inline_problems` (1 for a single call)
     uint32_t inline_tile_start[kInlineProblems + 1];   // first tile of each inline problem, then the tile count
-    uint32_t pad1[3];
+    uint32_t pad1[4];
     GemmProblem inline_problems[kInlineProblems];
 };
 

@@ -129,19 +129,6 @@ __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc]; `accumulate` == 0 overwrites D.
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                        uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t"
-        "}\n"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
 // The four MMAs of one pipeline stage in a single statement. A stage holds 128 bytes of K per row
 // (one swizzle span) and every MMA consumes 32 of them, so the operand start addresses advance by
 // 32 B >> 4 = 2 descriptor units per MMA. The 64-bit shared-memory descriptors are passed as their
@@ -338,23 +325,6 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t tmem_address, uint32_
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_address), "r"(columns)
                  : "memory");
 }
-
-#define SDXLQ_UMMA_PAIR(NAME, KIND)                                                                     \
-    __device__ __forceinline__ void NAME(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,            \
-                                         uint32_t idesc, uint32_t accumulate) {                         \
-        asm volatile(                                                                                   \
-            "{\n\t"                                                                                     \
-            ".reg .pred p;\n\t"                                                                         \
-            "setp.ne.b32 p, %4, 0;\n\t"                                                                 \
-            "tcgen05.mma.cta_group::2.kind::" KIND " [%0], %1, %2, %3, p;\n\t"                          \
-            "}\n"                                                                                       \
-            ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)                        \
-            : "memory");                                                                                \
-    }
-SDXLQ_UMMA_PAIR(umma_i8_pair, "i8")
-SDXLQ_UMMA_PAIR(umma_f8f6f4_pair, "f8f6f4")
-SDXLQ_UMMA_PAIR(umma_f16_pair, "f16")
-#undef SDXLQ_UMMA_PAIR
 
 // Completion of the pair's MMAs -> one arrival on the barrier at `cluster_address` (own or peer CTA).
 __device__ __forceinline__ void umma_commit_pair(uint32_t cluster_address) {
