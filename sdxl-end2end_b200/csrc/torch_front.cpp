@@ -3,7 +3,7 @@
 //
 // What bounds it: host time. A projection of few rows runs for 5 to 15 us on the GPU; checking its arguments,
 // allocating its output and filling a ctypes descriptor in Python cost more than that again. Measured per call
-// with its launches (B200 box): FP8 of two rows 15.3 -> 10.3 us, FP16 of 154 rows 11.1 -> 9.9 us (now the
+// with its launches (B200): FP8 of two rows 15.3 -> 10.3 us, FP16 of 154 rows 11.1 -> 9.9 us (now the
 // kernels), the ten calls of a transformer block's weight packing 113 -> 68 us.
 //
 // Every function answers with
